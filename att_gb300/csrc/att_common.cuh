@@ -140,6 +140,13 @@ __device__ __forceinline__ void red_add_f32(float *p, float v) {
     asm volatile("red.global.add.f32 [%0], %1;\n" ::"l"(p), "f"(v) : "memory");
 }
 
+// ---- programmatic dependent launch ----------------------------------------
+// griddep_launch: the dependent kernel may start once every CTA has called it
+// (or ended).  griddep_wait: returns when the kernel before has completed and
+// its writes are visible (at once in a kernel launched without the attribute).
+__device__ __forceinline__ void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // ---- mbarrier / TMA ---------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(bar), "r"(count) : "memory");

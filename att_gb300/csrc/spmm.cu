@@ -5,26 +5,25 @@
 // SpMM_sr_bcrs.forward_{fp16,tf32}_gnn[_acc] (gcn/SpMM/src/benchmark.cpp:35-335).
 //
 // Design (sm_103a):
-//  * One warp owns one work item = (part, chunk of FC features) at a time and
-//    walks its items in a persistent grid-stride sequence.  Each k-step is 16
-//    condensed columns: the 16 gathered X rows (FC features each) and the
-//    16 x W value block are copied global->shared with 16-byte cp.async into
-//    an S-stage ring; the producer cursor runs S-1 steps ahead of the
-//    consumer across item boundaries, so the gather stream never drains.
+//  * One CTA per SM; a warp owns one work item = (part, chunk of FC features) at
+//    a time and streams its condensed columns in chunks of 32: the gathered X
+//    rows (FC features each) and the value blocks are copied global->shared with
+//    16-byte cp.async ahead of the products and across item boundaries, so the
+//    gather stream never drains (spmm_stream.cuh).
 //  * The contraction is D[feature, row] += X^T[feature, col] * V[col, row]:
 //    M = 16 features, N = 8 window rows, K = 16 columns, so the sparse block
 //    is the dense B operand and the gathered rows are A.  ldmatrix.trans
 //    turns the row-major gathered X tile into the A fragment; the value tile
 //    feeds B through a plain ldmatrix.  fp32 accumulators stay in registers.
 //    (The reference uses m16n8k8 with fp16 accumulation; this accumulates in
-//    fp32.)  Shared rows are XOR-swizzled per 16-byte chunk so both ldmatrix
-//    forms are bank-conflict free.
-//  * TF32 runs m16n8k8 as a 3xTF32 split (hi*hi + hi*lo + lo*hi), which gives
-//    fp32-level accuracy at no cost on a gather-bound kernel.
+//    fp32.)
+//  * TF32 runs m16n8k8 as a 3xTF32 split (hi*hi + hi*lo + lo*hi): fp32-level
+//    accuracy.
 //  * Output: a part of an unsplit window stores its whole W-row tile with
 //    plain stores; parts of split windows add with red.global.add.f32.  A
-//    small pre-pass zeroes only rows that no unsplit part writes (split
-//    windows, windows without parts, trailing rows), so Y needs no memset.
+//    small pre-pass, which the kernel behind it overlaps, zeroes only rows that
+//    no unsplit part writes (split windows, windows without parts, trailing
+//    rows), so Y needs no memset.
 #include "att_common.cuh"
 
 #include <cuda.h>
@@ -50,12 +49,9 @@ struct PartInfo {
 // reads (the value tile of a 16-column step is read whole); a part that does
 // not is flagged and skipped instead of read past its end.
 template <int WIDE>
-__device__ __forceinline__ PartInfo part_info(const int32_t *__restrict__ rowptr, int64_t p,
-                                              int32_t *err) {
+__device__ __forceinline__ PartInfo part_check(int start, int e, int pend, int32_t *err) {
     PartInfo pi;
-    pi.start = __ldg(rowptr + 2 * p);
-    const int e = __ldg(rowptr + 2 * p + 1);
-    const int pend = __ldg(rowptr + 2 * p + 2);
+    pi.start = start;
     pi.nreal = e > pi.start ? e - pi.start : 0;
     if ((pi.start % WIDE) != 0 || (pend % WIDE) != 0 || pend < pi.start + pi.nreal) {
         if (err) atomicOr(err, 2);
@@ -63,6 +59,11 @@ __device__ __forceinline__ PartInfo part_info(const int32_t *__restrict__ rowptr
     }
     pi.nsteps = (pi.nreal + 15) >> 4;
     return pi;
+}
+template <int WIDE>
+__device__ __forceinline__ PartInfo part_info(const int32_t *__restrict__ rowptr, int64_t p,
+                                              int32_t *err) {
+    return part_check<WIDE>(__ldg(rowptr + 2 * p), __ldg(rowptr + 2 * p + 1), __ldg(rowptr + 2 * p + 2), err);
 }
 
 // XOR swizzle of the 16-byte chunk index within a shared row of `row_bytes`
@@ -72,205 +73,110 @@ __device__ __forceinline__ int swz(int r) {
     else return (r >> 1) & 3;  // 64-byte rows: two rows share a 128-byte bank window
 }
 
+}  // namespace
+}  // namespace att
+
+#include "spmm_stream.cuh"
+
+namespace att {
+namespace {
+
 // ---------------------------------------------------------------------------
 // 16-bit operand kernel (fp16 / bf16 values and features)
 // ---------------------------------------------------------------------------
-template <typename T, int W, int FC, int WIDE, int S = kStages>
-struct Cfg16 {
-    static constexpr int XROW = FC * 2;                 // bytes per gathered row in smem
-    static constexpr int XSTAGE = 16 * XROW;            // 16 rows per k-step
-    static constexpr int VSTAGE = 16 * W * 2;           // 16 cols x W rows
-    static constexpr int STAGE = XSTAGE + VSTAGE;
-    static constexpr int WARP_SMEM = S * STAGE;
-    static constexpr int SMEM = kWarps * WARP_SMEM;
-    static constexpr int CPR = FC / 8;                  // 16-byte chunks per row
-    static constexpr int RPP = 32 / CPR;                // rows per warp pass
-    static constexpr int MT = FC / 16;                  // m16 tiles
-    static constexpr int NT = W / 8;                    // n8 tiles
-    static constexpr int VCH = VSTAGE / 16;             // value chunks per step
-    // 8-row windows with <= 64 features: as many CTAs per SM as shared memory
-    // allows (228 KB per SM, 1 KB reserved per CTA; 8 for the default shape)
-    // bound the registers; other shapes keep the compiler's choice
-    static constexpr int MINB_RAW = (228 * 1024) / (SMEM + 1024);
-    static constexpr int MINB =
-        (W != 8 || FC > 64) ? 1 : (MINB_RAW < 1 ? 1 : (MINB_RAW > 8 ? 8 : MINB_RAW));
+// The chunk stream of spmm_stream.cuh; the lane layout and the contraction are
+// those described at the top of this file.
+template <int W, int FC, int WIDE, int S>
+struct Cfg16 : StreamCfg<FC * 2, 2, W, WIDE, S, (W == 16 ? (FC == 128 ? 12 : 16) : (FC == 32 ? 32 : 24))> {
+    static constexpr int NT = W / 8;   // n8 tiles
+    static constexpr int MT = FC / 16; // m16 tiles
 };
 
-// IT: index type of items and element offsets -- int32_t when every offset
-// into X, Y and the values fits (the common case: fewer instructions per
-// gathered row; the kernel is issue-bound), else int64_t.
-// FULL: F is a multiple of FC (every chunk whole; no per-feature bounds checks)
-template <typename T, int W, int FC, int WIDE, int S, typename IT, bool FULL>
-__global__ void __launch_bounds__(kThreads, (Cfg16<T, W, FC, WIDE, S>::MINB)) k_spmm16(
-    const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-    const T *__restrict__ val, const int32_t *__restrict__ win,
-    const int32_t *__restrict__ atomic, int64_t n_parts, const T *__restrict__ X, int64_t n_x_,
-    int64_t F_, int64_t ldx_, float *__restrict__ Y, int64_t m_out_, int64_t ldy_, int n_chunks,
-    int32_t *__restrict__ err) {
-    using C = Cfg16<T, W, FC, WIDE, S>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
-    const IT n_x = (IT)n_x_, F = (IT)F_, ldx = (IT)ldx_, m_out = (IT)m_out_, ldy = (IT)ldy_;
-    const IT n_items = (IT)(n_parts * n_chunks);
-    const IT stride = (IT)gridDim.x * kWarps;
-    const int gid = lane >> 2, tig = lane & 3;
-
-    // ---- producer cursor ----
-    IT p_item = (IT)blockIdx.x * kWarps + warp;
-    int p_step = 0, p_myc = -1;
-    PartInfo p_pi = {0, 0, 0};
-    int p_fc = 0;
-    auto p_load = [&]() {
-        while (p_item < n_items) {
-            const IT part = p_item / n_chunks;
-            p_fc = (int)(p_item - part * n_chunks);
-            p_pi = part_info<WIDE>(rowptr, part, err);
-            p_step = 0;
-            if (p_pi.nsteps > 0) return;
-            p_item += stride;
-        }
-    };
-    auto issue = [&](int stage) {
-        const uint32_t xs = sbase + stage * C::STAGE;
-        const uint32_t vs = xs + C::XSTAGE;
-        const int c0 = p_step * 16;
-        int myc = p_myc;  // loaded one step ahead
-        // valid ids are -1 (padding) .. n_x - 1; an id outside is flagged and
-        // gathered as padding (zeros) -- checked once per id, not per chunk
-        if ((uint64_t)(int64_t)(myc + 1) > (uint64_t)n_x) {
-            if (err) atomicOr(err, 1);
-            myc = -1;
-        }
-        const IT fbase = (IT)p_fc * FC;
-        const bool full = FULL || fbase + FC <= F;  // the whole chunk is inside F (uniform)
-        // CPR lanes copy one row's FC features per pass (whole 128-byte lines
-        // per instruction; spreading a row over lane pairs measured 2.4x
-        // slower on the 2.45M-node graph)
+// Products of 16 gathered rows (FC features; `xl`: the lane's ldmatrix.trans
+// address of feature tile 0) with their values' fragments.
+template <typename T, int NT, int FC>
+__device__ __forceinline__ void half_mma(float (&acc)[FC / 16][NT][4], uint32_t xl, const uint32_t (&b)[NT][2]) {
 #pragma unroll
-        for (int i = 0; i < 16 / C::RPP; ++i) {
-            const int r = i * C::RPP + lane / C::CPR;
-            const int ch = lane % C::CPR;
-            const int cidx = __shfl_sync(0xffffffffu, myc, r);
-            const IT f = fbase + ch * 8;
-            const bool ok = cidx >= 0 && (full || f < F);
-            // padding: src-size 0 fills zeros (the source stays X's base)
-            const IT off = ok ? (IT)cidx * ldx + f : (IT)0;
-            cp_async16(xs + r * C::XROW + ((ch ^ swz<C::XROW>(r)) << 4), X + off, ok ? 16 : 0);
-        }
+    for (int j = 0; j < FC / 16; ++j) {
+        uint32_t a[4];
+        ldsm_x4_trans((xl ^ ((j & 3) << 5)) + (j >> 2) * 128, a[0], a[1], a[2], a[3]);
 #pragma unroll
-        for (int q = lane; q < C::VCH; q += 32) {
-            const int e = q * 8;                       // element offset within the step's block run
-            const int blk = e / (W * WIDE);
-            const bool ok = c0 + blk * WIDE < p_pi.nreal;
-            const T *src = val + ((IT)(p_pi.start + c0) * W + e);
-            cp_async16(vs + q * 16, ok ? (const void *)src : (const void *)val, ok ? 16 : 0);
-        }
-    };
-    // column ids of the producer's position, fetched one step ahead so the
-    // load latency overlaps the consumer's work instead of stalling issue()
-    auto p_fetch = [&]() {
-        p_myc = -1;
-        if (p_item < n_items && p_step * 16 + (lane & 15) < p_pi.nreal)
-            p_myc = __ldg(col + p_pi.start + p_step * 16 + (lane & 15));
-    };
-    auto p_advance = [&]() {
-        if (++p_step >= p_pi.nsteps) {
-            p_item += stride;
-            p_load();
-        }
-        p_fetch();
-    };
-
-    p_load();
-    p_fetch();
-#pragma unroll
-    for (int s = 0; s < S - 1; ++s) {
-        if (p_item < n_items) {
-            issue(s);
-            p_advance();
-        }
-        cp_async_commit();
+        for (int t = 0; t < NT; ++t) mma_16816<T>(acc[j][t], a, b[t][0], b[t][1]);
     }
+}
 
-    // ---- consumer ----
+// S: chunk buffers per warp (two steps each)
+template <typename T, int W, int FC, int WIDE, int S, typename IT, bool FULL>
+__global__ void __launch_bounds__((Cfg16<W, FC, WIDE, S>::NW * 32), 1)
+    k_spmm16(const __grid_constant__ StreamArgs A, float *__restrict__ Y, int64_t m_out, int64_t ldy) {
+    using C = Cfg16<W, FC, WIDE, S>;
+    extern __shared__ __align__(128) unsigned char smem[];
+    __shared__ int queue;
+    const int lane = threadIdx.x & 31, warp = warp_uniform(threadIdx.x >> 5);
+    const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
+    const int gid = lane >> 2, tig = lane & 3;
+    // ldmatrix lanes: matrix q = lane / 8, row lane % 8
+    const int q = lane >> 3, rr = lane & 7;
+    const int xk = (q >> 1) * 8 + rr;
+    const uint32_t xlane = sbase + xk * C::XROW + (((q & 1) ^ swz<C::XROW>(xk)) << 4);
+    // 16-byte piece of the values: 8 columns (kb) of window row r
+    auto vpiece = [](int kb, int r) { return WIDE == 8 ? (kb * W + r) * 16 : (kb >> 1) * W * 32 + r * 32 + (kb & 1) * 16; };
+    // W 8: matrix q = columns 8 q ..; W 16: columns 8 (q & 1) .., rows 8 (q >> 1) .. of a half
+    const uint32_t vlane = sbase + C::VAL + (W == 8 ? vpiece(q, rr) : vpiece(q & 1, (q >> 1) * 8 + rr));
+
     float acc[C::MT][C::NT][4];
 #pragma unroll
     for (int j = 0; j < C::MT; ++j)
 #pragma unroll
         for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
 
-    int cstage = 0, pstage = S - 1;
-    for (IT c_item = (IT)blockIdx.x * kWarps + warp; c_item < n_items; c_item += stride) {
-        const IT part = c_item / n_chunks;
-        const int fc = (int)(c_item - part * n_chunks);
-        const PartInfo pi = part_info<WIDE>(rowptr, part, err);
-        for (int step = 0; step < pi.nsteps; ++step) {
-            cp_async_wait<S - 2>();
-            __syncwarp();
-            const uint32_t xs = sbase + cstage * C::STAGE;
-            const uint32_t vs = xs + C::XSTAGE;
-            // B fragments: value tile rows = window rows, 8 columns per matrix
-            uint32_t b[C::NT][2];
-            {
-                const int q = lane >> 3, rr = lane & 7;
-                if constexpr (C::NT == 2) {
-                    const int kb = q & 1, r = (q >> 1) * 8 + rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x4(vs + e * 2, b[0][0], b[0][1], b[1][0], b[1][1]);
-                } else {
-                    const int kb = q & 1, r = rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x2(vs + e * 2, b[0][0], b[0][1]);
-                }
-            }
+    Stream<C, 2, FC, IT, FULL> st(A, lane, warp, sbase, &queue);
+    while (st.more()) {
+        const Chunk c = st.next();
+        if (c.left > 0) {
+            uint32_t b[2][C::NT][2];
+            if constexpr (W == 8) {
+                ldsm_x4(vlane + st.rbuf, b[0][0][0], b[0][0][1], b[1][0][0], b[1][0][1]);
+            } else {
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const int q = lane >> 3, rr = lane & 7;
-                const int k = (q >> 1) * 8 + rr;
-                const int ch = 2 * j + (q & 1);
-                uint32_t a[4];
-                ldsm_x4_trans(xs + k * C::XROW + ((ch ^ swz<C::XROW>(k)) << 4), a[0], a[1], a[2],
-                              a[3]);
-#pragma unroll
-                for (int t = 0; t < C::NT; ++t) mma_16816<T>(acc[j][t], a, b[t][0], b[t][1]);
+                for (int h = 0; h < 2; ++h)
+                    ldsm_x4(vlane + st.rbuf + h * 32 * W, b[h][0][0], b[h][0][1], b[h][1][0], b[h][1][1]);
             }
-            __syncwarp();
-            if (p_item < n_items) {
-                issue(pstage);
-                p_advance();
-            }
-            cp_async_commit();
-            cstage = cstage + 1 == S ? 0 : cstage + 1;
-            pstage = pstage + 1 == S ? 0 : pstage + 1;
+            half_mma<T, C::NT, FC>(acc, xlane + st.rbuf, b[0]);
+            if (c.left > 16) half_mma<T, C::NT, FC>(acc, xlane + st.rbuf + C::HALF, b[1]);
         }
-        // ---- epilogue: the W x FC tile of this part ----
-        const int wrow = __ldg(win + part);
-        const bool add = __ldg(atomic + part) != 0;
-        const IT f0 = (IT)fc * FC;
-        const bool full = FULL || f0 + FC <= F;
+        st.release();
+        if (c.left > 32) continue;
+        // ---- the part's last chunk: its W x FC tile ----
+        const IT f0 = (IT)c.fc * FC + gid;
+        const bool add = c.win & 1;
+        if (add) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
-        for (int t = 0; t < C::NT; ++t) {
-            const IT r0 = (IT)wrow * W + t * 8 + 2 * tig;
+        for (int t = 0; t < C::NT; ++t)
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const IT fa = f0 + 16 * j + gid;
+            for (int h = 0; h < 2; ++h) {
+                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
+                float *dst = Y + (r * ldy + f0);
+                if (r < m_out) {
+                    // Y is written once: a streaming store leaves L2 to the X rows
+                    if (add) {
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const IT r = r0 + (h & 1);
-                    const IT f = fa + (h >> 1) * 8;
-                    if (r < m_out && (full || f < F)) {
-                        float *dst = Y + (r * ldy + f);
-                        // Y is written once: a streaming store leaves L2 to the X rows
-                        if (add) red_add_f32(dst, acc[j][t][h]);
-                        else __stcs(dst, acc[j][t][h]);
+                        for (int j = 0; j < 2 * C::MT; ++j)
+                            if (FULL || f0 + 8 * j < st.F) red_add_f32(dst + 8 * j, acc[j / 2][t][h + 2 * (j & 1)]);
+                    } else {
+#pragma unroll
+                        for (int j = 0; j < 2 * C::MT; ++j)
+                            if (FULL || f0 + 8 * j < st.F) __stcs(dst + 8 * j, acc[j / 2][t][h + 2 * (j & 1)]);
                     }
-                    acc[j][t][h] = 0.f;
                 }
             }
-        }
+#pragma unroll
+        for (int j = 0; j < C::MT; ++j)
+#pragma unroll
+            for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
     }
     cp_async_wait<0>();
+    griddep_wait();  // this kernel ends after the one before it
 }
 
 constexpr uint32_t kMaxPolls = 1u << 24;  // bounded mbarrier waits
@@ -683,105 +589,34 @@ __global__ void __launch_bounds__(kThreads) k_spmm16_tma(
 // ---------------------------------------------------------------------------
 // fp32 operand kernel: 3xTF32 m16n8k8
 // ---------------------------------------------------------------------------
-template <int W, int FC, int WIDE, int S = kStages>
-struct CfgTF32 {
-    static constexpr int XROW = FC * 4;
-    static constexpr int XSTAGE = 16 * XROW;
-    static constexpr int VSTAGE = 16 * W * 4;
-    static constexpr int STAGE = XSTAGE + VSTAGE;
-    static constexpr int WARP_SMEM = S * STAGE;
-    static constexpr int SMEM = kWarps * WARP_SMEM;
-    static constexpr int CPR = FC / 4;
-    static constexpr int RPP = 32 / CPR;
+// The chunk stream of spmm_stream.cuh.  Per 8-column k-step lane (gid, tig)
+// reads rows 2 tig and 2 tig + 1 (the MMA's k = tig and tig + 4: both operands
+// use this order) with 16-byte loads, conflict-free under the row swizzle;
+// each brings four features of one row, the m = gid and gid + 8 elements of
+// two feature tiles, so a tile's rows are features 4 gid + 2 v (+ 1) and a lane
+// ends up with four adjacent features of its window rows: one float4 store.
+// 169,343 nodes, mean degree 14, F = 100: 178 us, 9.4 TB/s into the SMs; with
+// one 4-byte load per fragment element in a per-step ring it took 369 us.
+template <int W, int FC, int WIDE, int S>
+struct CfgTF32 : StreamCfg<FC * 4, 4, W, WIDE, S, (W == 16 ? 12 : 20)> {
     static constexpr int MT = FC / 16;
     static constexpr int NT = W / 8;
-    static constexpr int VCH = VSTAGE / 16;
 };
 
-
-template <int W, int FC, int WIDE, int S>
-__global__ void __launch_bounds__(kThreads) k_spmm_tf32(
-    const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-    const float *__restrict__ val, const int32_t *__restrict__ win,
-    const int32_t *__restrict__ atomic, int64_t n_parts, const float *__restrict__ X, int64_t n_x,
-    int64_t F, int64_t ldx, float *__restrict__ Y, int64_t m_out, int64_t ldy, int n_chunks,
-    int32_t *__restrict__ err) {
+template <int W, int FC, int WIDE, int S, typename IT>
+__global__ void __launch_bounds__((CfgTF32<W, FC, WIDE, S>::NW * 32), 1)
+    k_spmm_tf32(const __grid_constant__ StreamArgs A, float *__restrict__ Y, int64_t m_out, int64_t ldy, int vec_out) {
     using C = CfgTF32<W, FC, WIDE, S>;
     extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int queue;
+    const int lane = threadIdx.x & 31, warp = warp_uniform(threadIdx.x >> 5);
     const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
     const unsigned char *sgen = smem + warp * C::WARP_SMEM;
-    const int64_t n_items = n_parts * n_chunks;
-    const int64_t stride = (int64_t)gridDim.x * kWarps;
     const int gid = lane >> 2, tig = lane & 3;
-
-    int64_t p_item = (int64_t)blockIdx.x * kWarps + warp;
-    int p_step = 0, p_fc = 0, p_myc = -1;
-    PartInfo p_pi = {0, 0, 0};
-    auto p_load = [&]() {
-        while (p_item < n_items) {
-            int64_t part = p_item / n_chunks;
-            p_fc = (int)(p_item - part * n_chunks);
-            p_pi = part_info<WIDE>(rowptr, part, err);
-            p_step = 0;
-            if (p_pi.nsteps > 0) return;
-            p_item += stride;
-        }
-    };
-    auto issue = [&](int stage) {
-        const uint32_t xs = sbase + stage * C::STAGE;
-        const uint32_t vs = xs + C::XSTAGE;
-        const int c0 = p_step * 16;
-        int myc = p_myc;  // loaded one step ahead
-        const int64_t fbase = (int64_t)p_fc * FC;
-#pragma unroll
-        for (int i = 0; i < 16 / C::RPP; ++i) {
-            const int r = i * C::RPP + lane / C::CPR;
-            const int ch = lane % C::CPR;
-            const int cidx = __shfl_sync(0xffffffffu, myc, r);
-            const int64_t f = fbase + ch * 4;
-            bool ok = cidx >= 0 && f < F;
-            if (cidx >= n_x || cidx < -1) {
-                if (err) atomicOr(err, 1);
-                ok = false;
-            }
-            const float *src = ok ? X + (int64_t)cidx * ldx + f : X;
-            cp_async16(xs + r * C::XROW + ((ch ^ ((r & 3) << 1)) << 4), src, ok ? 16 : 0);
-        }
-#pragma unroll
-        for (int q = lane; q < C::VCH; q += 32) {
-            const int e = q * 4;
-            const int blk = e / (W * WIDE);
-            const bool ok = c0 + blk * WIDE < p_pi.nreal;
-            const float *src = val + ((int64_t)(p_pi.start + c0) * W + e);
-            cp_async16(vs + q * 16, ok ? (const void *)src : (const void *)val, ok ? 16 : 0);
-        }
-    };
-    // column ids of the producer's position, fetched one step ahead so the
-    // load latency overlaps the consumer's work instead of stalling issue()
-    auto p_fetch = [&]() {
-        p_myc = -1;
-        if (p_item < n_items && p_step * 16 + (lane & 15) < p_pi.nreal)
-            p_myc = __ldg(col + p_pi.start + p_step * 16 + (lane & 15));
-    };
-    auto p_advance = [&]() {
-        if (++p_step >= p_pi.nsteps) {
-            p_item += stride;
-            p_load();
-        }
-        p_fetch();
-    };
-
-    p_load();
-    p_fetch();
-#pragma unroll
-    for (int s = 0; s < S - 1; ++s) {
-        if (p_item < n_items) {
-            issue(s);
-            p_advance();
-        }
-        cp_async_commit();
-    }
+    const int x0off = 2 * tig * C::XROW + ((gid ^ (2 * tig)) << 4);
+    const int x1off = (2 * tig + 1) * C::XROW + ((gid ^ (2 * tig + 1)) << 4);
+    // values of columns 2 tig, 2 tig + 1 (of a k-step) and window row gid
+    const int voff = C::VAL + 4 * ((2 * tig / WIDE * W + gid) * WIDE + 2 * tig % WIDE);
 
     float acc[C::MT][C::NT][4];
 #pragma unroll
@@ -789,81 +624,65 @@ __global__ void __launch_bounds__(kThreads) k_spmm_tf32(
 #pragma unroll
         for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
 
-    int cstage = 0, pstage = S - 1;
-    for (int64_t c_item = (int64_t)blockIdx.x * kWarps + warp; c_item < n_items; c_item += stride) {
-        const int64_t part = c_item / n_chunks;
-        const int fc = (int)(c_item - part * n_chunks);
-        const PartInfo pi = part_info<WIDE>(rowptr, part, err);
-        for (int step = 0; step < pi.nsteps; ++step) {
-            cp_async_wait<S - 2>();
-            __syncwarp();
-            const float *xsg = (const float *)(sgen + cstage * C::STAGE);
-            const float *vsg = (const float *)(sgen + cstage * C::STAGE + C::XSTAGE);
+    Stream<C, 4, FC, IT, false> st(A, lane, warp, sbase, &queue);
+    while (st.more()) {
+        const Chunk c = st.next();
+        const unsigned char *buf = sgen + st.rbuf;
+#pragma unroll 1
+        for (int ks = 0; 8 * ks < c.left && ks < 4; ++ks) {  // 8 columns
+            const unsigned char *xs = buf + ks * 8 * C::XROW;
+            uint32_t bh[C::NT][2], bl[C::NT][2];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {  // two k8 steps per 16-column stage
-                uint32_t bh[C::NT][2], bl[C::NT][2];
+            for (int t = 0; t < C::NT; ++t) {
+                const float2 v = *reinterpret_cast<const float2 *>(buf + voff + ks * 32 * W + t * 32 * WIDE);
+                split_tf32x3(v.x, bh[t][0], bl[t][0]);
+                split_tf32x3(v.y, bh[t][1], bl[t][1]);
+            }
 #pragma unroll
-                for (int t = 0; t < C::NT; ++t) {
+            for (int u = 0; u < C::MT / 2; ++u) {
+                const float4 r0 = *reinterpret_cast<const float4 *>(xs + x0off + 128 * u);
+                const float4 r1 = *reinterpret_cast<const float4 *>(xs + x1off + 128 * u);
+                const float x[2][4] = {{r0.x, r0.y, r1.x, r1.y}, {r0.z, r0.w, r1.z, r1.w}};
 #pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const int c = 8 * h + tig + 4 * u;
-                        const int r = t * 8 + gid;
-                        const float v = vsg[(c / WIDE) * W * WIDE + r * WIDE + c % WIDE];
-                        split_tf32x3(v, bh[t][u], bl[t][u]);
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < C::MT; ++j) {
+                for (int v = 0; v < 2; ++v) {
                     uint32_t ah[4], al[4];
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int k = 8 * h + tig + ((u >> 1) << 2);
-                        const int f = 16 * j + gid + ((u & 1) << 3);
-                        const int ch = f >> 2;
-                        const float x = xsg[k * FC + (((ch ^ ((k & 3) << 1))) << 2) + (f & 3)];
-                        split_tf32x3(x, ah[u], al[u]);
-                    }
+                    for (int k = 0; k < 4; ++k) split_tf32x3(x[v][k], ah[k], al[k]);
 #pragma unroll
                     for (int t = 0; t < C::NT; ++t) {
-                        mma_1688_tf32(acc[j][t], al[0], al[1], al[2], al[3], bh[t][0], bh[t][1]);
-                        mma_1688_tf32(acc[j][t], ah[0], ah[1], ah[2], ah[3], bl[t][0], bl[t][1]);
-                        mma_1688_tf32(acc[j][t], ah[0], ah[1], ah[2], ah[3], bh[t][0], bh[t][1]);
+                        float(&d)[4] = acc[2 * u + v][t];
+                        mma_1688_tf32(d, al[0], al[1], al[2], al[3], bh[t][0], bh[t][1]);
+                        mma_1688_tf32(d, ah[0], ah[1], ah[2], ah[3], bl[t][0], bl[t][1]);
+                        mma_1688_tf32(d, ah[0], ah[1], ah[2], ah[3], bh[t][0], bh[t][1]);
                     }
                 }
             }
-            __syncwarp();
-            if (p_item < n_items) {
-                issue(pstage);
-                p_advance();
-            }
-            cp_async_commit();
-            cstage = cstage + 1 == S ? 0 : cstage + 1;
-            pstage = pstage + 1 == S ? 0 : pstage + 1;
         }
-        const int wrow = __ldg(win + part);
-        const bool add = __ldg(atomic + part) != 0;
-        const int64_t f0 = (int64_t)fc * FC;
+        st.release();
+        if (c.left > 32) continue;
+        const IT f0 = (IT)c.fc * FC + 4 * gid;
+        const bool add = c.win & 1;
+        if (add) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
-        for (int t = 0; t < C::NT; ++t) {
-            const int64_t r0 = (int64_t)wrow * W + t * 8 + 2 * tig;
+        for (int t = 0; t < C::NT; ++t)
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const int64_t fa = f0 + 16 * j + gid;
+            for (int h = 0; h < 2; ++h) {
+                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
+                if (r >= m_out) continue;
+                float *dst = Y + (r * ldy + f0);
 #pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int64_t r = r0 + (h & 1);
-                    const int64_t f = fa + (h >> 1) * 8;
-                    if (r >= 0 && r < m_out && f < F) {
-                        float *dst = Y + r * ldy + f;
-                        if (add) red_add_f32(dst, acc[j][t][h]);
-                        else *dst = acc[j][t][h];
-                    }
-                    acc[j][t][h] = 0.f;
-                }
+                for (int u = 0; u < C::MT / 2; ++u)
+                    if (f0 + 32 * u < st.F)  // F is a multiple of 4
+                        put4(dst + 32 * u, add, vec_out, acc[2 * u][t][h], acc[2 * u][t][h + 2],
+                             acc[2 * u + 1][t][h], acc[2 * u + 1][t][h + 2]);
             }
-        }
+#pragma unroll
+        for (int j = 0; j < C::MT; ++j)
+#pragma unroll
+            for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
     }
     cp_async_wait<0>();
+    griddep_wait();  // this kernel ends after the one before it
 }
 
 // ---------------------------------------------------------------------------
@@ -1121,29 +940,17 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fp8(
 // each lane ends up owning two adjacent features of two window rows and
 // stores them as float2.  This removes the shared-memory round trip of the
 // fp16 tile (4 KB of shared traffic and four 16-byte stores per lane per
-// step) and lets one work item cover 128 features.
+// step) and lets one work item cover 128 features.  2.45M nodes, F = 128:
+// 1.27 ms on the chunk stream, 1.77 ms in a per-step ring (bound by issue).
 constexpr float kF8Shift = 32768.f;
 constexpr float kF8Unshift = 1.f / 32768.f;
 
-__device__ __forceinline__ bool f16_normal_or_zero(float x) {
-    const float a = fabsf(x);
-    return a == 0.f || (a >= 6.103515625e-05f && a <= 65504.f);
-}
+constexpr unsigned kF16Min = 0x38800000u, kF16Max = 0x477fe000u;  // 2^-14 and 65504 as fp32 bits
 
-template <int W, int FC, int S = kF8Stages>
-struct CfgF8R {
-    static constexpr int XROW = FC;              // bytes per gathered e4m3 row
-    static constexpr int XSTAGE = 16 * XROW;
-    static constexpr int VSTAGE = 16 * W * 2;
-    static constexpr int SSTAGE = 64;            // 16 fp32 scales
-    static constexpr int STAGE = XSTAGE + VSTAGE + SSTAGE;
-    static constexpr int WARP_SMEM = S * STAGE;
-    static constexpr int SMEM = kWarps * WARP_SMEM;
-    static constexpr int CPR = FC / 16;          // 16-byte chunks per row
-    static constexpr int RPP = 32 / CPR;         // rows per warp pass
+template <int W, int FC, int WIDE>
+struct CfgF8R : StreamCfg<FC, 2, W, WIDE, 2, (W == 16 ? 12 : (FC == 128 ? 20 : 24)), 128> {  // + the 32 row scales
     static constexpr int MT = FC / 16;           // 16-feature MMA tiles
     static constexpr int NT = W / 8;
-    static constexpr int VCH = VSTAGE / 16;
 };
 
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, __half2 s) {
@@ -1152,95 +959,23 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, __half2 s) {
 }
 
 template <int W, int FC, int WIDE, typename IT, bool FULL>
-__global__ void __launch_bounds__(kThreads) k_spmm_fp8r(
-    const int32_t *__restrict__ rowptr, const int32_t *__restrict__ col,
-    const __half *__restrict__ val, const int32_t *__restrict__ win,
-    const int32_t *__restrict__ atomic, int64_t n_parts, const uint8_t *__restrict__ X,
-    const float *__restrict__ xscale, int64_t n_x_, int64_t F_, int64_t ldx_, float *__restrict__ Y,
-    int64_t m_out_, int64_t ldy_, int n_chunks, int vec_out, int32_t *__restrict__ err) {
-    const IT n_x = (IT)n_x_, F = (IT)F_, ldx = (IT)ldx_, m_out = (IT)m_out_, ldy = (IT)ldy_;
-    using C = CfgF8R<W, FC>;
-    constexpr int S = kF8Stages;
+__global__ void __launch_bounds__((CfgF8R<W, FC, WIDE>::NW * 32), 1)
+    k_spmm_fp8r(const __grid_constant__ StreamArgs A, float *__restrict__ Y, int64_t m_out, int64_t ldy, int vec_out) {
+    using C = CfgF8R<W, FC, WIDE>;
     extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int queue;
+    const int lane = threadIdx.x & 31, warp = warp_uniform(threadIdx.x >> 5);
     const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
     const unsigned char *sgen = smem + warp * C::WARP_SMEM;
-    const IT n_items = (IT)(n_parts * n_chunks);
-    const IT stride = (IT)gridDim.x * kWarps;
     const int gid = lane >> 2, tig = lane & 3;
-
-    IT p_item = (IT)blockIdx.x * kWarps + warp;
-    int p_step = 0, p_fc = 0, p_myc = -1;
-    PartInfo p_pi = {0, 0, 0};
-    auto p_load = [&]() {
-        while (p_item < n_items) {
-            const IT part = p_item / n_chunks;
-            p_fc = (int)(p_item - part * n_chunks);
-            p_pi = part_info<WIDE>(rowptr, part, err);
-            p_step = 0;
-            if (p_pi.nsteps > 0) return;
-            p_item += stride;
-        }
-    };
-    auto issue = [&](int stage) {
-        const uint32_t xs = sbase + stage * C::STAGE;
-        const uint32_t vs = xs + C::XSTAGE;
-        const uint32_t ss = vs + C::VSTAGE;
-        const int c0 = p_step * 16;
-        int myc = p_myc;  // loaded one step ahead
-        if ((uint64_t)(int64_t)(myc + 1) > (uint64_t)n_x) {  // valid: -1 .. n_x - 1
-            if (err) atomicOr(err, 1);
-            myc = -1;
-        }
-        const IT fbase = (IT)p_fc * FC;
-        const bool full = FULL || fbase + FC <= F;
-#pragma unroll
-        for (int i = 0; i < 16 / C::RPP; ++i) {
-            const int r = i * C::RPP + lane / C::CPR;
-            const int ch = lane % C::CPR;
-            const int cidx = __shfl_sync(0xffffffffu, myc, r);
-            const IT f = fbase + ch * 16;
-            const bool ok = cidx >= 0 && (full || f < F);
-            const IT off = ok ? (IT)cidx * ldx + f : (IT)0;
-            cp_async16(xs + r * C::XROW + ((ch ^ swz<C::XROW>(r)) << 4), X + off, ok ? 16 : 0);
-        }
-#pragma unroll
-        for (int q = lane; q < C::VCH; q += 32) {
-            const int e = q * 8;
-            const int blk = e / (W * WIDE);
-            const bool ok = c0 + blk * WIDE < p_pi.nreal;
-            const __half *src = val + ((IT)(p_pi.start + c0) * W + e);
-            cp_async16(vs + q * 16, ok ? (const void *)src : (const void *)val, ok ? 16 : 0);
-        }
-        if (lane < 16) {
-            const bool ok = myc >= 0;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(ss + 4 * lane),
-                         "l"(ok ? xscale + myc : xscale), "r"(ok ? 4 : 0));
-        }
-    };
-    auto p_fetch = [&]() {
-        p_myc = -1;
-        if (p_item < n_items && p_step * 16 + (lane & 15) < p_pi.nreal)
-            p_myc = __ldg(col + p_pi.start + p_step * 16 + (lane & 15));
-    };
-    auto p_advance = [&]() {
-        if (++p_step >= p_pi.nsteps) {
-            p_item += stride;
-            p_load();
-        }
-        p_fetch();
-    };
-
-    p_load();
-    p_fetch();
-#pragma unroll
-    for (int s = 0; s < S - 1; ++s) {
-        if (p_item < n_items) {
-            issue(s);
-            p_advance();
-        }
-        cp_async_commit();
-    }
+    // ldmatrix lane roles: matrix mi = lane / 8 holds gathered rows
+    // (mi / 2) * 8 + lane % 8 and 16-feature piece (mi % 2) of a 32-feature pair
+    const int q = lane >> 3, rr = lane & 7;
+    const int lm_k = (q >> 1) * 8 + rr;
+    const uint32_t xlane = sbase + lm_k * C::XROW + (((q & 1) ^ swz<C::XROW>(lm_k)) << 4);
+    // value pieces as in k_spmm16
+    auto vpiece = [](int kb, int r) { return WIDE == 8 ? (kb * W + r) * 16 : (kb >> 1) * W * 32 + r * 32 + (kb & 1) * 16; };
+    const uint32_t vlane = sbase + C::VAL + vpiece(q & 1, (W == 16 ? (q >> 1) * 8 : 0) + rr);
 
     float acc[C::MT][C::NT][4];
 #pragma unroll
@@ -1248,38 +983,20 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fp8r(
 #pragma unroll
         for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
 
-    // ldmatrix lane roles: matrix mi = lane / 8 holds gathered rows
-    // (mi / 2) * 8 + lane % 8 and 16-feature chunk (mi % 2) of a 32-feature pair
-    const int lm_k = ((lane >> 4) << 3) + (lane & 7);
-    const int lm_h = (lane >> 3) & 1;
-    int cstage = 0, pstage = S - 1;
-    for (IT c_item = (IT)blockIdx.x * kWarps + warp; c_item < n_items; c_item += stride) {
-        const IT part = c_item / n_chunks;
-        const int fc = (int)(c_item - part * n_chunks);
-        const PartInfo pi = part_info<WIDE>(rowptr, part, nullptr);
-        for (int step = 0; step < pi.nsteps; ++step) {
-            cp_async_wait<S - 2>();
-            __syncwarp();
-            const uint32_t xs = sbase + cstage * C::STAGE;
-            const uint32_t vs = xs + C::XSTAGE;
-            const float *sc = (const float *)(sgen + cstage * C::STAGE + C::XSTAGE + C::VSTAGE);
+    Stream<C, 1, FC, IT, FULL> st(A, lane, warp, sbase, &queue);
+    while (st.more()) {
+        const Chunk c = st.next();
+        const float *scales = reinterpret_cast<const float *>(sgen + st.rbuf + C::EXT);
+#pragma unroll 1  // unrolled it spills at this register bound
+        for (int hf = 0; hf < 2 && 16 * hf < c.left; ++hf) {
+            uint32_t b[C::NT][2];
+            if constexpr (W == 16) ldsm_x4(vlane + st.rbuf + hf * 32 * W, b[0][0], b[0][1], b[1][0], b[1][1]);
+            else ldsm_x2(vlane + st.rbuf + hf * 32 * W, b[0][0], b[0][1]);
+            const uint32_t xl = xlane + st.rbuf + hf * C::HALF;
             // scale pairs of the gathered rows this lane's A fragments hold:
             // rows (2 tig, 2 tig + 1) and (8 + 2 tig, 9 + 2 tig)
-            const float2 s_lo = *reinterpret_cast<const float2 *>(sc + 2 * tig);
-            const float2 s_hi = *reinterpret_cast<const float2 *>(sc + 8 + 2 * tig);
-            uint32_t b[C::NT][2];
-            {
-                const int q = lane >> 3, rr = lane & 7;
-                if constexpr (C::NT == 2) {
-                    const int kb = q & 1, r = (q >> 1) * 8 + rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x4(vs + e * 2, b[0][0], b[0][1], b[1][0], b[1][1]);
-                } else {
-                    const int kb = q & 1, r = rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x2(vs + e * 2, b[0][0], b[0][1]);
-                }
-            }
+            const float2 s_lo = *reinterpret_cast<const float2 *>(scales + 16 * hf + 2 * tig);
+            const float2 s_hi = *reinterpret_cast<const float2 *>(scales + 16 * hf + 8 + 2 * tig);
             // The row scales go on the B fragment: b[t][0] holds the values of
             // gathered rows (2 tig, 2 tig + 1), b[t][1] of (8 + 2 tig, 9 + 2 tig),
             // exactly the rows of the lane's scale pairs.  V * s is multiplied
@@ -1288,114 +1005,99 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fp8r(
             // would be neither zero nor a normal fp16, the warp scales A
             // instead for that step (accumulators brought back to 1 * Y around
             // it, exact: powers of two).
+            const float sk[4] = {s_lo.x * kF8Shift, s_lo.y * kF8Shift, s_hi.x * kF8Shift, s_hi.y * kF8Shift};
             uint32_t bs[C::NT][2];
-            bool ok = true;
+            // magnitudes as integers order like the floats; 0 - 1 wraps, so a
+            // zero never is the smallest (and a NaN is above any finite value)
+            unsigned lo = ~0u, hi = 0;
 #pragma unroll
             for (int t = 0; t < C::NT; ++t) {
 #pragma unroll
                 for (int g = 0; g < 2; ++g) {
                     const float2 v = __half22float2(*reinterpret_cast<const __half2 *>(&b[t][g]));
-                    const float2 sg = g == 0 ? s_lo : s_hi;
-                    const float p0 = v.x * sg.x * kF8Shift, p1 = v.y * sg.y * kF8Shift;
-                    ok = ok && f16_normal_or_zero(p0) && f16_normal_or_zero(p1);
+                    const float p0 = v.x * sk[2 * g], p1 = v.y * sk[2 * g + 1];
+                    const unsigned m0 = __float_as_uint(p0) & 0x7fffffffu, m1 = __float_as_uint(p1) & 0x7fffffffu;
+                    lo = min(lo, min(m0 - 1, m1 - 1));
+                    hi = max(hi, max(m0, m1));
                     const __half2 hp = __floats2half2_rn(p0, p1);
                     bs[t][g] = *reinterpret_cast<const uint32_t *>(&hp);
                 }
             }
-            const bool bside = __all_sync(0xffffffffu, ok);
-            __half2 h_lo, h_hi;
-            if (!bside) {
-                h_lo = __floats2half2_rn(s_lo.x, s_lo.y);
-                h_hi = __floats2half2_rn(s_hi.x, s_hi.y);
+            const bool bside = __all_sync(0xffffffffu, lo >= kF16Min - 1 && hi <= kF16Max);
+            auto products = [&](auto scaled, __half2 h_lo, __half2 h_hi) {
+                constexpr bool kScaleA = decltype(scaled)::value;
 #pragma unroll
-                for (int j = 0; j < C::MT; ++j)
+                for (int jp = 0; jp < C::MT / 2; ++jp) {
+                    uint32_t R[4];  // (rows 0-7 | 8-15) x (tile 2jp | 2jp+1)
+                    ldsm_x4_trans(xl ^ (jp << 5), R[0], R[1], R[2], R[3]);
 #pragma unroll
-                    for (int t = 0; t < C::NT; ++t)
-#pragma unroll
-                        for (int q = 0; q < 4; ++q) acc[j][t][q] *= kF8Unshift;
-            }
-#pragma unroll
-            for (int jp = 0; jp < C::MT / 2; ++jp) {
-                const int ch = 2 * jp + lm_h;
-                uint32_t R[4];  // (rows 0-7 | 8-15) x (tile 2jp | 2jp+1)
-                ldsm_x4_trans(xs + lm_k * C::XROW + ((ch ^ swz<C::XROW>(lm_k)) << 4), R[0], R[1],
-                              R[2], R[3]);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    // bytes (f: c, f+1: c, f: c+1, f+1: c+1) -> (f: c, c+1 | f+1: c, c+1)
-                    const uint32_t p0 = __byte_perm(R[h], 0, 0x3120);      // rows 2tig, 2tig+1
-                    const uint32_t p1 = __byte_perm(R[h + 2], 0, 0x3120);  // rows 8+2tig, 9+2tig
-                    uint32_t a[4];
-                    a[0] = e4m3x2_to_f16x2((uint16_t)(p0 & 0xffffu));
-                    a[1] = e4m3x2_to_f16x2((uint16_t)(p0 >> 16));
-                    a[2] = e4m3x2_to_f16x2((uint16_t)(p1 & 0xffffu));
-                    a[3] = e4m3x2_to_f16x2((uint16_t)(p1 >> 16));
-                    if (bside) {
+                    for (int h = 0; h < 2; ++h) {
+                        // bytes (f: c, f+1: c, f: c+1, f+1: c+1) -> (f: c, c+1 | f+1: c, c+1)
+                        const uint32_t p0 = __byte_perm(R[h], 0, 0x3120);      // rows 2tig, 2tig+1
+                        const uint32_t p1 = __byte_perm(R[h + 2], 0, 0x3120);  // rows 8+2tig, 9+2tig
+                        uint32_t a[4];
+                        a[0] = e4m3x2_to_f16x2((uint16_t)(p0 & 0xffffu));
+                        a[1] = e4m3x2_to_f16x2((uint16_t)(p0 >> 16));
+                        a[2] = e4m3x2_to_f16x2((uint16_t)(p1 & 0xffffu));
+                        a[3] = e4m3x2_to_f16x2((uint16_t)(p1 >> 16));
+                        if constexpr (kScaleA) {
+                            a[0] = hmul2_u32(a[0], h_lo);
+                            a[1] = hmul2_u32(a[1], h_lo);
+                            a[2] = hmul2_u32(a[2], h_hi);
+                            a[3] = hmul2_u32(a[3], h_hi);
+                        }
 #pragma unroll
                         for (int t = 0; t < C::NT; ++t)
-                            mma_16816<__half>(acc[2 * jp + h][t], a, bs[t][0], bs[t][1]);
-                    } else {
-                        a[0] = hmul2_u32(a[0], h_lo);
-                        a[1] = hmul2_u32(a[1], h_lo);
-                        a[2] = hmul2_u32(a[2], h_hi);
-                        a[3] = hmul2_u32(a[3], h_hi);
-#pragma unroll
-                        for (int t = 0; t < C::NT; ++t)
-                            mma_16816<__half>(acc[2 * jp + h][t], a, b[t][0], b[t][1]);
+                            mma_16816<__half>(acc[2 * jp + h][t], a, kScaleA ? b[t][0] : bs[t][0],
+                                              kScaleA ? b[t][1] : bs[t][1]);
                     }
                 }
-            }
-            if (!bside) {
+            };
+            if (bside) {
+                products(std::false_type{}, __half2{}, __half2{});
+            } else {
 #pragma unroll
                 for (int j = 0; j < C::MT; ++j)
 #pragma unroll
                     for (int t = 0; t < C::NT; ++t)
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) acc[j][t][q] *= kF8Shift;
+                        for (int k = 0; k < 4; ++k) acc[j][t][k] *= kF8Unshift;
+                products(std::true_type{}, __floats2half2_rn(s_lo.x, s_lo.y), __floats2half2_rn(s_hi.x, s_hi.y));
+#pragma unroll
+                for (int j = 0; j < C::MT; ++j)
+#pragma unroll
+                    for (int t = 0; t < C::NT; ++t)
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) acc[j][t][k] *= kF8Shift;
             }
-            __syncwarp();
-            if (p_item < n_items) {
-                issue(pstage);
-                p_advance();
-            }
-            cp_async_commit();
-            cstage = cstage + 1 == S ? 0 : cstage + 1;
-            pstage = pstage + 1 == S ? 0 : pstage + 1;
         }
+        st.release();
+        if (c.left > 32) continue;
         // epilogue: tile j, lane -> features f0 + 16 j + 2 gid (+1), window
         // rows t * 8 + 2 tig (+1); F is a multiple of 16, so both features of
         // a pair are inside F together
-        const int wrow = __ldg(win + part);
-        const bool add = __ldg(atomic + part) != 0;
-        const IT f0 = (IT)fc * FC;
+        const bool add = c.win & 1;
+        if (add) griddep_wait();  // the window's rows are zeroed by then
+        const IT f0 = (IT)c.fc * FC + 2 * gid;
 #pragma unroll
-        for (int t = 0; t < C::NT; ++t) {
-            const IT r0 = (IT)wrow * W + t * 8 + 2 * tig;
+        for (int t = 0; t < C::NT; ++t)
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const IT f = f0 + 16 * j + 2 * gid;
+            for (int h = 0; h < 2; ++h) {
+                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
+                if (r >= m_out) continue;
+                float *dst = Y + (r * ldy + f0);
 #pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const IT r = r0 + h;
-                    const float v0 = acc[j][t][h] * kF8Unshift, v1 = acc[j][t][h + 2] * kF8Unshift;
-                    if (r < m_out && (FULL || f < F)) {
-                        float *dst = Y + (r * ldy + f);
-                        if (add) {
-                            red_add_f32(dst, v0);
-                            red_add_f32(dst + 1, v1);
-                        } else if (vec_out) {
-                            *reinterpret_cast<float2 *>(dst) = make_float2(v0, v1);
-                        } else {
-                            dst[0] = v0;
-                            dst[1] = v1;
-                        }
-                    }
-                    acc[j][t][h] = acc[j][t][h + 2] = 0.f;
-                }
+                for (int j = 0; j < C::MT; ++j)
+                    if (FULL || f0 + 16 * j < st.F)
+                        put2(dst + 16 * j, add, vec_out, acc[j][t][h] * kF8Unshift, acc[j][t][h + 2] * kF8Unshift);
             }
-        }
+#pragma unroll
+        for (int j = 0; j < C::MT; ++j)
+#pragma unroll
+            for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
     }
     cp_async_wait<0>();
+    griddep_wait();  // this kernel ends after the one before it
 }
 
 // ---------------------------------------------------------------------------
@@ -1460,6 +1162,27 @@ __device__ __forceinline__ bool job_small(const att_spmm_job *j) {
            j->F < lim && j->ldx < lim && j->ldy < lim;
 }
 
+template <typename T, int W, int FC, int WIDE, int S = kStages>
+struct CfgB {
+    static constexpr int XROW = FC * 2;                 // bytes per gathered row in smem
+    static constexpr int XSTAGE = 16 * XROW;            // 16 rows per k-step
+    static constexpr int VSTAGE = 16 * W * 2;           // 16 cols x W rows
+    static constexpr int STAGE = XSTAGE + VSTAGE;
+    static constexpr int WARP_SMEM = S * STAGE;
+    static constexpr int SMEM = kWarps * WARP_SMEM;
+    static constexpr int CPR = FC / 8;                  // 16-byte chunks per row
+    static constexpr int RPP = 32 / CPR;                // rows per warp pass
+    static constexpr int MT = FC / 16;                  // m16 tiles
+    static constexpr int NT = W / 8;                    // n8 tiles
+    static constexpr int VCH = VSTAGE / 16;             // value chunks per step
+    // 8-row windows with <= 64 features: as many CTAs per SM as shared memory
+    // allows (228 KB per SM, 1 KB reserved per CTA; 8 for the default shape)
+    // bound the registers; other shapes keep the compiler's choice
+    static constexpr int MINB_RAW = (228 * 1024) / (SMEM + 1024);
+    static constexpr int MINB =
+        (W != 8 || FC > 64) ? 1 : (MINB_RAW < 1 ? 1 : (MINB_RAW > 8 ? 8 : MINB_RAW));
+};
+
 // 8 CTAs per SM (64 registers): like k_spmm16, throughput follows resident warps
 template <int W, int FC, int WIDE, int S>
 __global__ void __launch_bounds__(kThreads, 8) k_spmm16_batched(const att_spmm_job *__restrict__ jobs,
@@ -1467,7 +1190,7 @@ __global__ void __launch_bounds__(kThreads, 8) k_spmm16_batched(const att_spmm_j
                                                                 int32_t *__restrict__ err) {
     static_assert(kRing >= S + 2, "item ring too small");
     using T = __half;
-    using C = Cfg16<T, W, FC, WIDE, S>;
+    using C = CfgB<T, W, FC, WIDE, S>;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ int ring[kWarps][kRing];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1827,24 +1550,25 @@ __global__ void k_empty_scatter(const int32_t *__restrict__ win, int64_t P, int6
     if (w == n_windows - 1) counts[3] = scanned[w] + empty;
 }
 
-// Outputs up to this size are zeroed whole before the SpMM kernel (one
-// memset, a few microseconds); larger ones by k_zero_uncovered.
-constexpr size_t kZeroAllBytes = 32ull << 20;
-
 // Zeroes the rows of Y that no unsplit part stores (windows whose parts add
-// with red.add, windows without parts, rows past the last window), before
-// the SpMM kernel.  Thread per part, plus one thread for the end: the first
-// part of each window zeroes the windows between the previous part's window
-// and its own, and its own window when that window is split; the extra
-// thread zeroes the windows after the last part's.  No searches: every
-// thread reads at most two window ids and one flag, coalesced.  The warp
-// zeroes each lane's rows together.
+// with red.add, windows without parts, rows past the last window) for the SpMM
+// kernel behind it.  Eight lanes per part, plus one group for the end: the
+// first part of each window zeroes the windows between the previous part's
+// window and its own, and its own window when that window is split; the extra
+// group zeroes the windows after the last part's.  No searches: every group
+// reads at most two window ids and one flag.  A gap of many windows (a graph
+// with long runs of empty rows) is shared by the whole warp.  The SpMM kernel
+// is launched as this one's programmatic dependent, so it gathers meanwhile
+// and waits only before its first addition (or its end); with the two in
+// sequence, this pass was 8 of 54 us on the 169,343-node graph and 27 us of
+// 1,770 on the 2.45M-node one.
 __global__ void k_zero_uncovered(const int32_t *__restrict__ win, const int32_t *__restrict__ atomic,
                                  int64_t n_parts, int W, float *__restrict__ Y, int64_t m_out,
-                                 int64_t F, int64_t ldy) {
-    const int lane = threadIdx.x & 31;
+                                 int64_t F, int64_t ldy, int vec) {
+    griddep_launch();
+    const int lane = threadIdx.x & 31, sub = lane & 7;
     const int64_t n_w = (m_out + W - 1) / W;
-    const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 3;
     int64_t g0 = 0, g1 = 0, own = -1;  // gap [g0, g1) and the own window to zero
     if (p < n_parts) {
         const int64_t w = __ldg(win + p);
@@ -1861,19 +1585,26 @@ __global__ void k_zero_uncovered(const int32_t *__restrict__ win, const int32_t 
     g0 = g0 < 0 ? 0 : g0;
     g1 = g1 > n_w ? n_w : g1;
     if (own >= n_w) own = -1;
-    unsigned m = __ballot_sync(0xffffffffu, g1 > g0 || own >= 0);
+    // lane `i` of `n` zeroes its share of the rows of windows [w0, w1)
+    auto zero = [&](int64_t w0, int64_t w1, int i, int n) {
+        const int64_t r1 = w1 * W < m_out ? w1 * W : m_out;
+        for (int64_t r = w0 * W; r < r1; ++r) {
+            float *row = Y + r * ldy;
+            if (vec)
+                for (int64_t f = 4 * i; f < F; f += 4 * n)
+                    *reinterpret_cast<float4 *>(row + f) = make_float4(0.f, 0.f, 0.f, 0.f);
+            else
+                for (int64_t f = i; f < F; f += n) row[f] = 0.f;
+        }
+    };
+    if (own >= 0) zero(own, own + 1, sub, 8);
+    const bool large = g1 - g0 > 32;
+    if (g1 > g0 && !large) zero(g0, g1, sub, 8);
+    unsigned m = __ballot_sync(0xffffffffu, large && sub == 0);
     while (m) {
         const int l = __ffs(m) - 1;
         m &= m - 1;
-        const int64_t lg0 = __shfl_sync(0xffffffffu, g0, l), lg1 = __shfl_sync(0xffffffffu, g1, l);
-        const int64_t lown = __shfl_sync(0xffffffffu, own, l);
-        for (int pass = 0; pass < 2; ++pass) {
-            const int64_t w0 = pass == 0 ? lg0 : lown, w1 = pass == 0 ? lg1 : lown + 1;
-            if (w1 <= w0 || w0 < 0) continue;
-            const int64_t r1 = w1 * W < m_out ? w1 * W : m_out;
-            for (int64_t r = w0 * W; r < r1; ++r)
-                for (int64_t f = lane; f < F; f += 32) Y[r * ldy + f] = 0.f;
-        }
+        zero(__shfl_sync(0xffffffffu, g0, l), __shfl_sync(0xffffffffu, g1, l), lane, 32);
     }
 }
 
@@ -1894,33 +1625,61 @@ int prepare(K kernel, int smem) {
     return cuda_status(e, "cudaFuncSetAttribute");
 }
 
-template <typename T, int W, int FC, int WIDE, int S = kStages>
+// Launches a kernel that may start while the one before it on the stream (one
+// that calls griddep_launch) still runs; it calls griddep_wait before it
+// touches what that one writes.
+template <typename... P, typename... Q>
+int launch_dependent(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t st, const char *what,
+                     const Q &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), what);
+}
+
+// A kernel as a type: instantiations that share a function type still get their
+// own dynamic shared memory opt-in (the attribute is set once per kernel).
+template <auto K>
+struct KernelOf {
+    static constexpr auto value = K;
+    static int prepared(int smem) {
+        static std::once_flag once;
+        static int prep = ATT_OK;
+        std::call_once(once, [&] { prep = prepare(K, smem); });
+        return prep;
+    }
+};
+
+template <typename T, int W, int FC, int WIDE, int S>
 int launch16(const int32_t *rowptr, const int32_t *col, const void *val, const int32_t *win,
              const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
              int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, cudaStream_t st) {
-    using C = Cfg16<T, W, FC, WIDE, S>;
+    using C = Cfg16<W, FC, WIDE, S>;
     const int n_chunks = (int)((F + FC - 1) / FC);
     const int64_t items = n_parts * n_chunks;
     if (items == 0) return ATT_OK;
-    // 32-bit indices when every element offset stays below 2^31: X rows
-    // (n_x * ldx), Y rows (m_out * ldy) and items (plus one grid stride of
-    // overshoot); value offsets are below 2^31 by the format's own limit
+    // 32-bit items (plus one grid stride of overshoot) and row pitch of X;
+    // offsets into X, Y and the values are 64-bit either way
     const int64_t lim = INT32_MAX - (1 << 22);
-    const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
-    auto run = [&](auto kernel) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
+    const bool small = ldx * (int64_t)sizeof(T) < lim && F < lim && items < lim;
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
-        const int grid = occupancy_grid(kernel, C::SMEM, items);
-        kernel<<<grid, kThreads, C::SMEM, st>>>(rowptr, col, (const T *)val, win, atomic, n_parts,
-                                                (const T *)X, n_x, F, ldx, Y, m_out, ldy, n_chunks,
-                                                err);
-        return launch_status("k_spmm16");
+        const int grid = (int)(items < sm_count() ? items : sm_count());
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, err};
+        return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm16", A, Y, m_out, ldy);
     };
-    if (small && F % FC == 0) return run(k_spmm16<T, W, FC, WIDE, S, int32_t, true>);
-    if (small) return run(k_spmm16<T, W, FC, WIDE, S, int32_t, false>);
-    return run(k_spmm16<T, W, FC, WIDE, S, int64_t, false>);
+    if (small && F % FC == 0) return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int32_t, true>>{});
+    if (small) return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int32_t, false>>{});
+    return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int64_t, false>>{});
 }
 
 template <typename T, int S>
@@ -1934,38 +1693,40 @@ int launch16_bulk(const int32_t *rowptr, const int32_t *col, const void *val, co
     if (items == 0) return ATT_OK;
     const int64_t lim = INT32_MAX - (1 << 22);
     const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
-    auto run = [&](auto kernel) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] { prep = prepare(kernel, SMEM); });
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = decltype(k)::prepared(SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = occupancy_grid(kernel, SMEM, items);
         kernel<<<grid, kThreads, SMEM, st>>>(rowptr, col, (const T *)val, win, atomic, n_parts,
                                              (const T *)X, n_x, F, ldx, Y, m_out, ldy, n_chunks, err);
         return launch_status("k_spmm16_bulk");
     };
-    if (small) return run(k_spmm16_bulk<T, S, int32_t>);
-    return run(k_spmm16_bulk<T, S, int64_t>);
+    if (small) return run(KernelOf<k_spmm16_bulk<T, S, int32_t>>{});
+    return run(KernelOf<k_spmm16_bulk<T, S, int64_t>>{});
 }
 
-template <int W, int FC, int WIDE, int S = kStages>
+template <int W, int FC, int WIDE, int S>
 int launch_tf32(const int32_t *rowptr, const int32_t *col, const void *val, const int32_t *win,
                 const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
                 int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, cudaStream_t st) {
     using C = CfgTF32<W, FC, WIDE, S>;
-    auto kernel = k_spmm_tf32<W, FC, WIDE, S>;
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
-    if (prep != ATT_OK) return prep;
     const int n_chunks = (int)((F + FC - 1) / FC);
     const int64_t items = n_parts * n_chunks;
     if (items == 0) return ATT_OK;
-    const int grid = occupancy_grid(kernel, C::SMEM, items);
-    kernel<<<grid, kThreads, C::SMEM, st>>>(rowptr, col, (const float *)val, win, atomic, n_parts,
-                                            (const float *)X, n_x, F, ldx, Y, m_out, ldy, n_chunks,
-                                            err);
-    return launch_status("k_spmm_tf32");
+    const int64_t lim = INT32_MAX - (1 << 22);  // as in launch16
+    const bool small = ldx * 4 < lim && F < lim && items < lim;
+    const int vec_out = ldy % 4 == 0 && ((uintptr_t)Y & 15) == 0;
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = decltype(k)::prepared(C::SMEM);
+        if (prep != ATT_OK) return prep;
+        const int grid = (int)(items < sm_count() ? items : sm_count());
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, err};
+        return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_tf32", A, Y, m_out, ldy, vec_out);
+    };
+    if (small) return run(KernelOf<k_spmm_tf32<W, FC, WIDE, S, int32_t>>{});
+    return run(KernelOf<k_spmm_tf32<W, FC, WIDE, S, int64_t>>{});
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
@@ -2022,14 +1783,14 @@ constexpr int kTmaStages = 5;
 // threads.
 //  * spmm_gather: row-gather mechanism of the 16-bit kernel, 0 = cp.async
 //    (default), 1 = TMA tile::gather4, 2 = cp.async.bulk per row.
-//  * spmm_stages / spmm_fc: ring depth of the 16-bit cp.async kernel (2, 3,
-//    4) and features per work item for F > 64 (64 or 128).  Measured on the
-//    2.45M-node graph (F = 128): throughput follows resident warps per SM,
-//    not the depth of each warp's ring.
+//  * spmm_stages / spmm_fc: chunk buffers per warp of the 16-bit kernel (2, 3:
+//    two; 4: three) and features per work item for F > 64 (64 or 128).  169,343
+//    nodes, F = 128: 64 features x 2 buffers 78 us, x 3 83; 128 x 2 74, x 3 84;
+//    on the 2.45M-node graph 64 x 2 is the faster one.
 //  * spmm_fp8: 1 = A fragments dequantized in registers (k_spmm_fp8r, 128
 //    features per item when F > 64), 0 = through an fp16 shared tile
 //    (k_spmm_fp8).
-//  * spmm_tf32: fp32-feature (3xTF32) kernel shape 0..3.
+//  * spmm_tf32: fp32-feature (3xTF32) kernel shape 0..3 (dispatch_fc32).
 enum SpmmOpt { kOptGather = 0, kOptStages, kOptFc, kOptFp8, kOptTf32, kNumOpts };
 const char *const kOptNames[kNumOpts] = {"spmm_gather", "spmm_stages", "spmm_fc", "spmm_fp8",
                                          "spmm_tf32"};
@@ -2069,10 +1830,9 @@ int launch_fp8(const int32_t *rowptr, const int32_t *col, const void *val, const
     if (items == 0) return ATT_OK;
     const int64_t lim = INT32_MAX - (1 << 22);
     const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
-    auto run = [&](auto kernel) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = occupancy_grid(kernel, C::SMEM, items);
         kernel<<<grid, kThreads, C::SMEM, st>>>(rowptr, col, (const __half *)val, win, atomic,
@@ -2080,8 +1840,8 @@ int launch_fp8(const int32_t *rowptr, const int32_t *col, const void *val, const
                                                 Y, m_out, ldy, n_chunks, err);
         return launch_status("k_spmm_fp8");
     };
-    if (small) return run(k_spmm_fp8<W, FC, WIDE, int32_t>);
-    return run(k_spmm_fp8<W, FC, WIDE, int64_t>);
+    if (small) return run(KernelOf<k_spmm_fp8<W, FC, WIDE, int32_t>>{});
+    return run(KernelOf<k_spmm_fp8<W, FC, WIDE, int64_t>>{});
 }
 
 template <int W, int FC, int WIDE>
@@ -2089,27 +1849,24 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
                 const int32_t *atomic, int64_t n_parts, const void *X, const float *xscale,
                 int64_t n_x, int64_t F, int64_t ldx, float *Y, int64_t m_out, int64_t ldy,
                 int32_t *err, cudaStream_t st) {
-    using C = CfgF8R<W, FC>;
+    using C = CfgF8R<W, FC, WIDE>;
     const int n_chunks = (int)((F + FC - 1) / FC);
     const int64_t items = n_parts * n_chunks;
     if (items == 0) return ATT_OK;
-    const int64_t lim = INT32_MAX - (1 << 22);
-    const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
+    const int64_t lim = INT32_MAX - (1 << 22);  // as in launch16
+    const bool small = ldx < lim && F < lim && items < lim;
     const int vec_out = (ldy % 2 == 0 && ((uintptr_t)Y & 7) == 0) ? 1 : 0;
-    auto run = [&](auto kernel) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
-        const int grid = occupancy_grid(kernel, C::SMEM, items);
-        kernel<<<grid, kThreads, C::SMEM, st>>>(rowptr, col, (const __half *)val, win, atomic,
-                                                n_parts, (const uint8_t *)X, xscale, n_x, F, ldx,
-                                                Y, m_out, ldy, n_chunks, vec_out, err);
-        return launch_status("k_spmm_fp8r");
+        const int grid = (int)(items < sm_count() ? items : sm_count());
+        const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, err};
+        return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_fp8r", A, Y, m_out, ldy, vec_out);
     };
-    if (small && F % FC == 0) return run(k_spmm_fp8r<W, FC, WIDE, int32_t, true>);
-    if (small) return run(k_spmm_fp8r<W, FC, WIDE, int32_t, false>);
-    return run(k_spmm_fp8r<W, FC, WIDE, int64_t, false>);
+    if (small && F % FC == 0) return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int32_t, true>>{});
+    if (small) return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int32_t, false>>{});
+    return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int64_t, false>>{});
 }
 
 template <typename T, int W, int WIDE>
@@ -2128,7 +1885,7 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
                                                          n_x, F, ldx, Y, m_out, ldy, err, st);
     }
     if (F <= 32)
-        return launch16<T, W, 32, WIDE>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
+        return launch16<T, W, 32, WIDE, 2>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
                                         m_out, ldy, err, st);
     if constexpr (W == 8 && WIDE == 8) {
         if (opt(kOptGather) == 2 && (F <= 64 || opt(kOptFc) == 64))
@@ -2139,13 +1896,11 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
     return launch16<T, W, FCv, WIDE, Sv>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, \
                                          Y, m_out, ldy, err, st)
     if (F <= 64 || opt(kOptFc) == 64) {
-        if (opt(kOptStages) == 2) ATT_L16S(64, 2);
-        if (opt(kOptStages) == 4) ATT_L16S(64, 4);
-        ATT_L16S(64, 3);
+        if (opt(kOptStages) == 4) ATT_L16S(64, 3);
+        ATT_L16S(64, 2);
     }
-    if (opt(kOptStages) == 2) ATT_L16S(128, 2);
-    if (opt(kOptStages) == 4) ATT_L16S(128, 4);
-    ATT_L16S(128, 3);
+    if (opt(kOptStages) == 4) ATT_L16S(128, 3);
+    ATT_L16S(128, 2);
 #undef ATT_L16S
 }
 
@@ -2157,14 +1912,15 @@ int dispatch_fc32(const int32_t *rowptr, const int32_t *col, const void *val, co
 #define ATT_LTF(FCv, Sv)                                                                        \
     return launch_tf32<W, FCv, WIDE, Sv>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, \
                                          Y, m_out, ldy, err, st)
-    // shapes (features per item x ring depth): 0 = 64 x 4, 1 = 32 x 3,
-    // 2 = 32 x 4, 3 = 64 x 2 (F <= 32 always takes 32-feature items)
+    // shapes (features per item x chunk buffers): 0, 3 = 64 x 2, 1 = 32 x 2,
+    // 2 = 32 x 3 (F <= 32 always takes 32-feature items).  169,343 nodes, mean
+    // degree 14, us for shapes 0, 1, 2: F 64 104, 115, 123; F 100 200, 211, 225;
+    // F 128 181, 201, 215
     if (F <= 32 || opt(kOptTf32) == 1 || opt(kOptTf32) == 2) {
-        if (opt(kOptTf32) == 1) ATT_LTF(32, 3);
-        ATT_LTF(32, 4);
+        if (opt(kOptTf32) == 2) ATT_LTF(32, 3);
+        ATT_LTF(32, 2);
     }
-    if (opt(kOptTf32) == 3) ATT_LTF(64, 2);
-    ATT_LTF(64, 4);
+    ATT_LTF(64, 2);
 #undef ATT_LTF
 }
 
@@ -2190,15 +1946,11 @@ extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *v
     cudaStream_t st = (cudaStream_t)stream;
     if (m_out == 0 || F == 0) return ATT_OK;
     int s = ATT_OK;
-    if ((size_t)m_out * (size_t)ldy * sizeof(float) <= kZeroAllBytes) {
-        // a small Y: zeroing all of it costs less than finding what to zero
-        ATT_CUDA(cudaMemset2DAsync(Y, (size_t)ldy * sizeof(float), 0, (size_t)F * sizeof(float),
-                                   (size_t)m_out, st),
-                 "zero Y");
-    } else {
-        const int64_t threads = n_parts + 1;
+    {
+        const int64_t threads = (n_parts + 1) * 8;
+        const int vec = F % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)Y & 15) == 0;
         k_zero_uncovered<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-            window_of_part, atomic, n_parts, window, Y, m_out, F, ldy);
+            window_of_part, atomic, n_parts, window, Y, m_out, F, ldy, vec);
         s = launch_status("k_zero_uncovered");
         if (s != ATT_OK) return s;
     }
@@ -2375,7 +2127,7 @@ extern "C" int att_host_device_pointer(const void *host, void **device) {
 }
 
 extern "C" size_t att_spmm_batched_grid(void) {
-    using C = Cfg16<__half, 8, 64, 8, 3>;
+    using C = CfgB<__half, 8, 64, 8, 3>;
     auto kernel = k_spmm16_batched<8, 64, 8, 3>;
     if (prepare(kernel, C::SMEM) != ATT_OK) return 0;
     int per_sm = 0;
@@ -2389,7 +2141,7 @@ extern "C" int att_spmm_batched(const att_spmm_job *jobs, int64_t *header, int64
     ATT_CHECK(window == 8 && wide == 8, ATT_ERR_UNSUPPORTED,
               "the batched SpMM takes the (8-row, 8-wide) fp16 format");
     ATT_CHECK(jobs && header && grid > 0, ATT_ERR_INVALID, "null table or empty grid");
-    using C = Cfg16<__half, 8, 64, 8, 3>;
+    using C = CfgB<__half, 8, 64, 8, 3>;
     auto kernel = k_spmm16_batched<8, 64, 8, 3>;
     static std::once_flag once;
     static int prep = ATT_OK;

@@ -70,12 +70,13 @@ enum att_dtype {
  *                  1 = TMA tile::gather4 row gathers (F >= 64),
  *                  2 = one cp.async.bulk per gathered row (8-row windows,
  *                      8-wide blocks, 64-feature chunks).
- *   "spmm_stages": ring depth of the 16-bit cp.async kernel (2, 3, 4).
+ *   "spmm_stages": prefetch depth of the 16-bit cp.async kernel: 2 and 3 (the
+ *                  default) two 32-column chunk buffers per warp, 4 three.
  *   "spmm_fc":     features per work item for F > 64 (64, the default, or 128).
  *   "spmm_fp8":    FP8 feature kernel: 1 = dequantized in registers (default),
  *                  0 = dequantized through an fp16 shared-memory tile.
- *   "spmm_tf32":   fp32-feature (3xTF32) kernel, features per item x ring
- *                  depth: 0 = 64 x 4 (default), 1 = 32 x 3, 2 = 32 x 4, 3 = 64 x 2. */
+ *   "spmm_tf32":   fp32-feature (3xTF32) kernel, features per item x chunk
+ *                  buffers: 0 and 3 = 64 x 2 (default 0), 1 = 32 x 2, 2 = 32 x 3. */
 ATT_API int att_set_option(const char *key, int value);
 ATT_API int att_set_thread_option(const char *key, int value);
 ATT_API int att_get_option(const char *key, int *value);
