@@ -22,6 +22,7 @@
 #include "att_common.cuh"
 
 #include <mutex>
+#include <type_traits>
 
 namespace att {
 namespace {
@@ -40,6 +41,15 @@ template <>
 __device__ __forceinline__ float ld_f<float>(const void *p, int64_t i) {
     return ((const float *)p)[i];
 }
+
+template <typename T>
+__device__ __forceinline__ T cvt_f(float v);
+template <>
+__device__ __forceinline__ __half cvt_f<__half>(float v) { return __float2half_rn(v); }
+template <>
+__device__ __forceinline__ __nv_bfloat16 cvt_f<__nv_bfloat16>(float v) { return __float2bfloat16_rn(v); }
+template <>
+__device__ __forceinline__ float cvt_f<float>(float v) { return v; }
 
 __device__ __forceinline__ float ld_any(const void *p, int dt, int64_t i) {
     if (dt == ATT_F16) return ld_f<__half>(p, i);
@@ -70,6 +80,75 @@ __global__ void k_node_scores(const void *__restrict__ X, int xdt, int64_t H, in
         acc += ld_any(X, xdt, h * xsh + m * xsm + f) * ld_any(a, adt, h * ash + f);
     acc = warp_sum(acc);
     if (lane == 0) s[h * ssh + m] = acc;
+}
+
+// 8 consecutive values as fp32
+template <typename T>
+__device__ __forceinline__ void ld8(float (&w)[8], const T *p) {
+    if constexpr (sizeof(T) == 2) {
+        const uint4 v = *reinterpret_cast<const uint4 *>(p);
+        const T *x = reinterpret_cast<const T *>(&v);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) w[k] = ld_f<T>(x, k);
+    } else {
+        const float4 a = *reinterpret_cast<const float4 *>(p), b = *reinterpret_cast<const float4 *>(p + 4);
+        w[0] = a.x, w[1] = a.y, w[2] = a.z, w[3] = a.w, w[4] = b.x, w[5] = b.y, w[6] = b.z, w[7] = b.w;
+    }
+}
+
+// The same sums in the same order for 16-bit rows of NF x 32 features, 4 lanes
+// per row with 16-byte loads: lane s holds features 8 s + k + 32 i, so its eight
+// partial sums over i are those of lanes 8 s + k above; lanes s ^ 2 and s ^ 1
+// exchange them (steps 16 and 8 of the warp sum), the last three steps are its
+// own.  Bound by the read of X (87 MB at 169,343 nodes x 4 heads x 64 features):
+// 110 -> 19 us.
+template <typename T, typename AT, int NF>
+__global__ void __launch_bounds__(256) k_node_scores_vec(const T *__restrict__ X, int64_t H, int64_t M, int64_t xsh,
+                                                         int64_t xsm, const AT *__restrict__ a, int64_t ash,
+                                                         float *__restrict__ s, int64_t ssh) {
+    const int sub = threadIdx.x & 3;
+    const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const bool ok = row < H * M;
+    const int64_t h = ok ? row / M : 0, m = ok ? row - h * M : 0;
+    float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (ok) {
+#pragma unroll
+        for (int i = 0; i < NF; ++i) {
+            float x[8], w[8];
+            ld8<T>(x, X + h * xsh + m * xsm + 32 * i + sub * 8);
+            ld8<AT>(w, a + h * ash + 32 * i + sub * 8);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] += x[k] * w[k];
+        }
+    }
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) t[k] += __shfl_xor_sync(0xffffffffu, t[k], o);
+    const float v = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+    if (ok && sub == 0) s[h * ssh + m] = v;
+}
+
+template <typename AT>
+bool node_scores_vec(const void *X, int x_dtype, int64_t H, int64_t M, int64_t F, int64_t xsh, int64_t xsm,
+                     const AT *a, int64_t ash, float *s, int64_t ssh, cudaStream_t st) {
+    if ((x_dtype != ATT_F16 && x_dtype != ATT_BF16) || (F != 32 && F != 64 && F != 128) || xsh % 8 || xsm % 8 ||
+        ash % 8 || (((uintptr_t)X | (uintptr_t)a) & 15))
+        return false;
+    const unsigned grid = (unsigned)((H * M * 4 + 255) / 256);
+    auto run = [&](auto *x, auto nf) {
+        using T = std::remove_pointer_t<decltype(x)>;
+        k_node_scores_vec<T, AT, decltype(nf)::value>
+            <<<grid, 256, 0, st>>>((const T *)X, H, M, xsh, xsm, a, ash, s, ssh);
+    };
+    auto with = [&](auto *x) {
+        if (F == 32) run(x, std::integral_constant<int, 1>{});
+        else if (F == 64) run(x, std::integral_constant<int, 2>{});
+        else run(x, std::integral_constant<int, 4>{});
+    };
+    if (x_dtype == ATT_F16) with((__half *)nullptr);
+    else with((__nv_bfloat16 *)nullptr);
+    return true;
 }
 
 // s0[h][m] = X[h][m] . a0[h] and s1[h][m] = X[h][m] . a1[h] in one pass over X
@@ -161,6 +240,135 @@ __global__ void k_slot_edges(SlotEdgeArgs A) {
     }
 }
 
+// The quad-layout forms (4-column sub-blocks, 8-row windows: every caller of the
+// drop-ins) of the three map operators.  One warp per part with all heads
+// inside: a block is 32 slots, so lane (r, c) = (lane / 4, lane % 4) meets row r
+// of the window in every block -- no divisions, one accumulator per head, the
+// map read once for all heads (it is the largest input: 81 MB against 20 MB of
+// edge values at 169,343 nodes) and four blocks in flight.  That graph, 4 heads:
+// row sums 534 -> 99 us, slot scores 486 -> SE_US, dense values 205 -> 66
+// against a warp (or thread) per part and head with runtime divisions.
+constexpr int kQuad = 4;
+constexpr int kQUnroll = 4;
+
+// part p's window and the number of its quad blocks
+struct QuadPart {
+    int64_t start;  // first condensed column
+    int n, win;
+};
+__device__ __forceinline__ QuadPart quad_part(const int32_t *__restrict__ rowptr, const int32_t *__restrict__ win,
+                                              int64_t p) {
+    const int s = rowptr[2 * p], e = rowptr[2 * p + 1];
+    return {s, e > s ? (e - s + kQuad - 1) / kQuad : 0, win[p]};
+}
+
+template <int HB>
+__global__ void __launch_bounds__(256) k_slot_edges_quad(SlotEdgeArgs A) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= A.n_parts) return;
+    const QuadPart q = quad_part(A.rowptr, A.win, p);
+    const int64_t row = (int64_t)q.win * 8 + (lane >> 2);
+    const int32_t *map = A.map + q.start * 8 + lane;
+    const int32_t *col = A.col + q.start + (lane & 3);
+    for (int64_t h0 = 0; h0 < A.H; h0 += HB) {
+        float rv[HB];
+#pragma unroll
+        for (int k = 0; k < HB; ++k) {
+            rv[k] = 0.f;
+            if (h0 + k < A.H && row < A.n_nodes)
+                rv[k] = A.mode == 0 ? A.s0[(h0 + k) * A.ssh + row]
+                                    : ld_any(A.g, A.gdt, (h0 + k) * A.gsh + row * A.gsn);
+        }
+        for (int b = 0; b < q.n; b += kQUnroll) {
+            int32_t e[kQUnroll], c[kQUnroll];
+#pragma unroll
+            for (int u = 0; u < kQUnroll; ++u) {
+                e[u] = b + u < q.n ? __ldg(map + (b + u) * 32) : -1;
+                c[u] = A.mode == 0 && b + u < q.n ? __ldg(col + (b + u) * kQuad) : -1;
+            }
+#pragma unroll
+            for (int u = 0; u < kQUnroll; ++u) {
+                if (e[u] < 0) continue;
+                const bool ok = c[u] >= 0 && c[u] < A.n_nodes;
+#pragma unroll
+                for (int k = 0; k < HB; ++k)
+                    if (h0 + k < A.H)
+                        st_any(A.out, A.odt, (h0 + k) * A.osh + (int64_t)e[u] * A.ose,
+                               ok ? rv[k] + __ldg(A.s1 + (h0 + k) * A.ssh + c[u]) : rv[k]);
+            }
+        }
+    }
+}
+
+// OW consecutive columns of one window row per thread: OW / 4 map quads of 16
+// bytes in, OW values of each head out (one 16-byte store for 16-bit values of
+// width 8 and fp32 values of width 4)
+template <typename VT, typename OT, int OW>
+__global__ void __launch_bounds__(256) k_gather_slots_quad(const int32_t *__restrict__ map, int64_t n_rows,
+                                                           const VT *__restrict__ vals, int64_t vsh, int64_t vse,
+                                                           int64_t H, OT *__restrict__ out, int64_t osh) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;  // block t / 8, window row t % 8
+    if (t >= n_rows) return;
+    int32_t e[OW];
+#pragma unroll
+    for (int k = 0; k < OW / 4; ++k) {
+        const int4 m = __ldg(reinterpret_cast<const int4 *>(map) + ((t >> 3) * (OW / 4) + k) * 8 + (t & 7));
+        e[4 * k] = m.x;
+        e[4 * k + 1] = m.y;
+        e[4 * k + 2] = m.z;
+        e[4 * k + 3] = m.w;
+    }
+    for (int64_t h = 0; h < H; ++h) {
+        alignas(16) OT v[OW];
+#pragma unroll
+        for (int k = 0; k < OW; ++k)
+            v[k] = e[k] >= 0 ? cvt_f<OT>(ld_f<VT>(vals, h * vsh + (int64_t)e[k] * vse)) : cvt_f<OT>(0.f);
+        static_assert(sizeof(v) == 16, "one store");
+        *reinterpret_cast<uint4 *>(out + h * osh + t * OW) = *reinterpret_cast<const uint4 *>(v);
+    }
+}
+
+template <int HB>
+__global__ void __launch_bounds__(256) k_rowsum_slots_quad(
+    const int32_t *__restrict__ rowptr, const int32_t *__restrict__ map, const int32_t *__restrict__ win,
+    const int32_t *__restrict__ atomic, int64_t n_parts, const void *vals, int vdt, int64_t vsh, int64_t vse,
+    int64_t H, float *out, int64_t osh, int64_t osm, int64_t m_out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (p >= n_parts) return;
+    const QuadPart q = quad_part(rowptr, win, p);
+    const int32_t *mp = map + q.start * 8 + lane;
+    const int64_t row = (int64_t)q.win * 8 + (lane >> 2);
+    const bool add = atomic[p] != 0;
+    for (int64_t h0 = 0; h0 < H; h0 += HB) {
+        float acc[HB];
+#pragma unroll
+        for (int k = 0; k < HB; ++k) acc[k] = 0.f;
+        for (int b = 0; b < q.n; b += kQUnroll) {
+            int32_t e[kQUnroll];
+#pragma unroll
+            for (int u = 0; u < kQUnroll; ++u) e[u] = b + u < q.n ? __ldg(mp + (b + u) * 32) : -1;
+#pragma unroll
+            for (int u = 0; u < kQUnroll; ++u)
+                if (e[u] >= 0)
+#pragma unroll
+                    for (int k = 0; k < HB; ++k)
+                        if (h0 + k < H) acc[k] += ld_any(vals, vdt, (h0 + k) * vsh + (int64_t)e[u] * vse);
+        }
+#pragma unroll
+        for (int k = 0; k < HB; ++k) {
+            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 2);
+            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 1);
+            if ((lane & 3) == 0 && h0 + k < H && row >= 0 && row < m_out) {
+                float *dst = out + (h0 + k) * osh + row * osm;
+                if (add) red_add_f32(dst, acc[k]);
+                else *dst = acc[k];
+            }
+        }
+    }
+}
+
 // ---- dense block values through the map ------------------------------------------
 // out is in the layout of block width out_wide, the map in that of map_wide
 // (W, map_wide and out_wide are powers of two, given as log2); heads on y
@@ -181,6 +389,19 @@ __global__ void k_gather_slots(const int32_t *__restrict__ map, int64_t n_slots,
         const float v = e >= 0 ? ld_any(vals, vdt, h * vsh + (int64_t)e * vse) : 0.f;
         st_any(out, odt, h * osh + s, v);
     }
+}
+
+// ---- block-width-`wide` slot map -> quad layout ----------------------------------
+// One 16-byte piece (4 columns of a window row) per thread, both ways; bound by
+// the two passes over the map (81 MB at 169,343 nodes and 8-row windows: 28 us, the torch index arithmetic it replaces 1,000).
+__global__ void __launch_bounds__(256) k_map_to_quad(const int4 *__restrict__ map, int64_t n4, int W, int wide4,
+                                                     int4 *__restrict__ out) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= n4) return;
+    // piece (quad q, row r); its block holds wide4 quads of W rows
+    const int64_t blk = t / (W * wide4);
+    const int in = (int)(t - blk * (W * wide4)), q = in / W, r = in - q * W;
+    out[t] = __ldg(map + blk * (W * wide4) + r * wide4 + q);
 }
 
 // ---- row sums through the map -----------------------------------------------------------
@@ -609,6 +830,15 @@ extern "C" int att_node_scores(const void *X, int x_dtype, int64_t n_heads, int6
     const int64_t warps = n_heads * n_nodes;
     if (warps == 0) return ATT_OK;
     ATT_CHECK(X && a && scores, ATT_ERR_INVALID, "null pointer");
+    const cudaStream_t st = (cudaStream_t)stream;
+    auto vec = [&](auto *v) {
+        using AT = std::remove_const_t<std::remove_pointer_t<decltype(v)>>;
+        return node_scores_vec<AT>(X, x_dtype, n_heads, n_nodes, F, x_stride_h, x_stride_n, v, a_stride_h, scores,
+                                   s_stride_h, st);
+    };
+    if (a_dtype == ATT_F32 ? vec((const float *)a)
+                           : a_dtype == ATT_F16 ? vec((const __half *)a) : vec((const __nv_bfloat16 *)a))
+        return launch_status("k_node_scores_vec");
     k_node_scores<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
         X, x_dtype, n_heads, n_nodes, F, x_stride_h, x_stride_n, a, a_dtype, a_stride_h, scores,
         s_stride_h);
@@ -675,6 +905,12 @@ extern "C" int att_slot_edges(const int32_t *rowptr, const int32_t *col, const i
     SlotEdgeArgs A{rowptr, col, map, window_of_part, n_parts, window, wide, mode, s0, s1,
                    s_stride_h, g, g_dtype, g_stride_h, g_stride_n, out, out_dtype, out_stride_h,
                    out_stride_e, n_heads, n_nodes};
+    if (window == 8 && wide == kQuad) {
+        const unsigned grid = (unsigned)((n_parts * 32 + 255) / 256);
+        if (n_heads == 1) k_slot_edges_quad<1><<<grid, 256, 0, (cudaStream_t)stream>>>(A);
+        else k_slot_edges_quad<4><<<grid, 256, 0, (cudaStream_t)stream>>>(A);
+        return launch_status("k_slot_edges_quad");
+    }
     k_slot_edges<<<(unsigned)((warps * 32 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(A);
     return launch_status("k_slot_edges");
 }
@@ -743,12 +979,54 @@ extern "C" int att_gather_slot_values(const int32_t *map, int64_t n_slots, int w
     ATT_CHECK(n_heads < 65536, ATT_ERR_UNSUPPORTED, "too many heads");
     if (n_slots == 0 || n_heads == 0) return ATT_OK;
     ATT_CHECK(map && vals && out, ATT_ERR_INVALID, "null pointer");
+    // one 16-byte store per thread and head: 16-bit values in 8-column blocks,
+    // fp32 in 4-column ones, from a quad map of 8-row windows
+    if (window == 8 && map_wide == kQuad && ((uintptr_t)map & 15) == 0 && ((uintptr_t)out & 15) == 0) {
+        const cudaStream_t st = (cudaStream_t)stream;
+        auto run = [&](auto *o, auto ow, auto *v) {
+            using OT = std::remove_pointer_t<decltype(o)>;
+            using VT = std::remove_pointer_t<decltype(v)>;
+            constexpr int OW = decltype(ow)::value;
+            const int64_t rows = n_slots / OW;
+            k_gather_slots_quad<VT, OT, OW><<<(unsigned)((rows + 255) / 256), 256, 0, st>>>(
+                map, rows, (const VT *)vals, v_stride_h, v_stride_e, n_heads, o, out_stride_h);
+            return launch_status("k_gather_slots_quad");
+        };
+        auto with = [&](auto *v) {
+            if (out_dtype == ATT_F16) return run((__half *)out, std::integral_constant<int, 8>{}, v);
+            if (out_dtype == ATT_BF16) return run((__nv_bfloat16 *)out, std::integral_constant<int, 8>{}, v);
+            return run((float *)out, std::integral_constant<int, 4>{}, v);
+        };
+        const bool fits = out_dtype == ATT_F32 ? out_wide == 4 && out_stride_h % 4 == 0
+                                               : out_wide == 8 && out_stride_h % 8 == 0;
+        if (fits && (n_slots >> 2) < ((int64_t)1 << 38)) {
+            if (v_dtype == ATT_F16) return with((__half *)nullptr);
+            if (v_dtype == ATT_BF16) return with((__nv_bfloat16 *)nullptr);
+            if (v_dtype == ATT_F32) return with((float *)nullptr);
+        }
+    }
     const int64_t want = (n_slots + 255) / 256, cap = (int64_t)sm_count() * 16;
     const dim3 grid((unsigned)(want < cap ? want : cap), (unsigned)n_heads);
     k_gather_slots<<<grid, 256, 0, (cudaStream_t)stream>>>(map, n_slots, lw, lmw, low, vals,
                                                           v_dtype, v_stride_h, v_stride_e, out,
                                                           out_dtype, out_stride_h);
     return launch_status("k_gather_slots");
+}
+
+extern "C" int att_map_to_quad(const int32_t *map, int64_t n_slots, int window, int wide, int32_t *out,
+                               void *stream) {
+    clear_error();
+    ATT_CHECK(window > 0 && wide >= 4 && wide % 4 == 0, ATT_ERR_UNSUPPORTED,
+              "blocks must be a multiple of 4 columns wide, got %d", wide);
+    ATT_CHECK(n_slots >= 0 && n_slots % ((int64_t)window * wide) == 0, ATT_ERR_INVALID,
+              "slot count is not a whole number of blocks");
+    if (n_slots == 0) return ATT_OK;
+    ATT_CHECK(map && out && map != out, ATT_ERR_INVALID, "null pointer, or a conversion in place");
+    ATT_CHECK((((uintptr_t)map | (uintptr_t)out) & 15) == 0, ATT_ERR_UNSUPPORTED, "maps must be 16-byte aligned");
+    const int64_t n4 = n_slots / 4;
+    k_map_to_quad<<<(unsigned)((n4 + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+        (const int4 *)map, n4, window, wide / 4, (int4 *)out);
+    return launch_status("k_map_to_quad");
 }
 
 extern "C" int att_rowsum(const int32_t *rowptr, const int32_t *map,
@@ -771,6 +1049,18 @@ extern "C" int att_rowsum(const int32_t *rowptr, const int32_t *map,
     const int64_t warps = n_parts * n_heads;
     if (warps == 0) return ATT_OK;
     ATT_CHECK(rowptr && map && window_of_part && atomic && vals, ATT_ERR_INVALID, "null pointer");
+    if (window == 8 && wide == kQuad) {
+        const unsigned qgrid = (unsigned)((n_parts * 32 + 255) / 256);
+        if (n_heads == 1)
+            k_rowsum_slots_quad<1><<<qgrid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, vals, v_dtype,
+                                                          v_stride_h, v_stride_e, n_heads, out, out_stride_h,
+                                                          out_stride_n, m_out);
+        else
+            k_rowsum_slots_quad<4><<<qgrid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, vals, v_dtype,
+                                                          v_stride_h, v_stride_e, n_heads, out, out_stride_h,
+                                                          out_stride_n, m_out);
+        return launch_status("k_rowsum_slots_quad");
+    }
     const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
     if (window == 8)
         k_rowsum_slots<8><<<grid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, wide,

@@ -26,6 +26,11 @@ def map_to_quad(map_std, window, wide):
     if wide == QUAD or map_std is None or map_std.numel() == 0:
         return map_std
     n = map_std.numel()
+    if (map_std.is_cuda and map_std.dtype == torch.int32 and map_std.is_contiguous() and wide % QUAD == 0
+            and n % (window * wide) == 0 and map_std.data_ptr() % 16 == 0):
+        out = torch.empty_like(map_std)
+        _lib.call("att_map_to_quad", _p(map_std), n, window, wide, _p(out), _stream())
+        return out
     s = torch.arange(n, device=map_std.device, dtype=torch.int64)
     blk, inb = s // (window * QUAD), s % (window * QUAD)
     r, g = inb // QUAD, blk * QUAD + inb % QUAD

@@ -289,6 +289,12 @@ ATT_API int att_gather_slot_values(const int32_t *map, int64_t n_slots, int wind
                    int64_t v_stride_h, int64_t v_stride_e, int64_t n_heads,
                    void *out, int out_dtype, int64_t out_stride_h, void *stream);
 
+/* Slot map of block width `wide` (a multiple of 4) -> the quad layout (4-column
+ * blocks) of the same slots; map and out are different 16-byte aligned arrays.
+ * (No counterpart in the reference, whose GAT map layout is not known.) */
+ATT_API int att_map_to_quad(const int32_t *map, int64_t n_slots, int window, int wide, int32_t *out,
+                   void *stream);
+
 /* Row sums of per-edge values through the map: out[h][i] = sum over slots of
  * row i of vals[h][map[s]] (spmm_*_{h_m,m_h}_rowsum, test_spmm_h_m_ones.py:45-68;
  * mgat_conv.py:126-132).  Every row < m_out is written (fp32). */
