@@ -109,7 +109,7 @@ struct StreamCfg {
     static constexpr int IDS = S * BUF;
     static constexpr int WARP_SMEM = IDS + 128;
     static constexpr int FIT = (227 * 1024 - 16) / WARP_SMEM;
-    static constexpr int NW = FIT < MAXW ? FIT : MAXW;
+    static constexpr int NW = (FIT < MAXW ? FIT : MAXW) / 4 * 4;  // as many on each of the four schedulers
     static constexpr int SMEM = NW * WARP_SMEM;
     static constexpr int CPR = XROW / 16;               // 16-byte pieces (copying lanes) per row
     static constexpr int RPL = CPR / 2;                 // rows per copying lane and half
