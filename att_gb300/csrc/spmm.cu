@@ -39,7 +39,6 @@ namespace {
 
 constexpr int kWarps = 4;
 constexpr int kThreads = kWarps * 32;
-constexpr int kStages = 4;
 
 struct PartInfo {
     int start, nreal, nsteps;
@@ -1132,27 +1131,6 @@ __device__ __forceinline__ int64_t find_prefix(const att_spmm_job *__restrict__ 
     return lo;
 }
 
-// Condensed-column run of parts [p0, p1) of one window.  At least one step
-// (an item whose run is empty -- only a malformed part -- streams one step
-// of zeros and stores zeros).
-template <int WIDE>
-__device__ __forceinline__ PartInfo group_info(const int32_t *__restrict__ rowptr, int64_t p0,
-                                               int64_t p1, int32_t *err) {
-    PartInfo pi;
-    pi.start = __ldg(rowptr + 2 * p0);
-    const int e = __ldg(rowptr + 2 * (p1 - 1) + 1);
-    const int pend = __ldg(rowptr + 2 * p1);
-    pi.nreal = e > pi.start ? e - pi.start : 0;
-    if ((pi.start % WIDE) != 0 || (pend % WIDE) != 0 || pend < pi.start + pi.nreal) {
-        if (err) atomicOr(err, 2);
-        pi.nreal = 0;
-    }
-    pi.nsteps = pi.nreal > 0 ? (pi.nreal + 15) >> 4 : 1;
-    return pi;
-}
-
-constexpr int kRing = 8;  // >= S + 2 items in flight per warp
-
 // A job's element offsets (X rows, Y rows, partial slots) fit in 31 bits:
 // the batched kernel computes them in 32-bit arithmetic and skips (error bit
 // 8) a job that does not fit instead of addressing it.
@@ -1162,227 +1140,261 @@ __device__ __forceinline__ bool job_small(const att_spmm_job *j) {
            j->F < lim && j->ldx < lim && j->ldy < lim;
 }
 
-template <typename T, int W, int FC, int WIDE, int S = kStages>
-struct CfgB {
-    static constexpr int XROW = FC * 2;                 // bytes per gathered row in smem
-    static constexpr int XSTAGE = 16 * XROW;            // 16 rows per k-step
-    static constexpr int VSTAGE = 16 * W * 2;           // 16 cols x W rows
-    static constexpr int STAGE = XSTAGE + VSTAGE;
-    static constexpr int WARP_SMEM = S * STAGE;
-    static constexpr int SMEM = kWarps * WARP_SMEM;
-    static constexpr int CPR = FC / 8;                  // 16-byte chunks per row
-    static constexpr int RPP = 32 / CPR;                // rows per warp pass
-    static constexpr int MT = FC / 16;                  // m16 tiles
-    static constexpr int NT = W / 8;                    // n8 tiles
-    static constexpr int VCH = VSTAGE / 16;             // value chunks per step
-    // 8-row windows with <= 64 features: as many CTAs per SM as shared memory
-    // allows (228 KB per SM, 1 KB reserved per CTA; 8 for the default shape)
-    // bound the registers; other shapes keep the compiler's choice
-    static constexpr int MINB_RAW = (228 * 1024) / (SMEM + 1024);
-    static constexpr int MINB =
-        (W != 8 || FC > 64) ? 1 : (MINB_RAW < 1 ? 1 : (MINB_RAW > 8 ? 8 : MINB_RAW));
-};
+// The chunk stream of spmm_stream.cuh over the job table: the same cursors, with
+// an item's pointers (X, values, ids of its job) beside its chunk, and two more
+// stages ahead of the fetch cursor because an item is found through the table
+// (job, group, part).  Items are drawn in increasing order, so a warp's job
+// search goes forward from its last job.
+using CfgBatch = StreamCfg<128, 2, 8, 8, 2, 20>;
 
-// 8 CTAs per SM (64 registers): like k_spmm16, throughput follows resident warps
-template <int W, int FC, int WIDE, int S>
-__global__ void __launch_bounds__(kThreads, 8) k_spmm16_batched(const att_spmm_job *__restrict__ jobs,
-                                                                int64_t *__restrict__ header,
-                                                                int32_t *__restrict__ err) {
-    static_assert(kRing >= S + 2, "item ring too small");
-    using T = __half;
-    using C = CfgB<T, W, FC, WIDE, S>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    __shared__ int ring[kWarps][kRing];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
-    const int64_t n_jobs = header[0];
-    const int n_fixed = (int)gridDim.x * kWarps;
-    if (header[1] > (int64_t)INT32_MAX - n_fixed - 1) {  // items must be 32-bit
-        if (err && threadIdx.x == 0 && blockIdx.x == 0) atomicOr(err, 8);
-        return;
+struct BatchStream {
+    using C = CfgBatch;
+    static constexpr int FC = 64, W = 8;
+    struct Work {
+        int start, left;       // first condensed column, real columns left in the group
+        int fc;                // feature chunk, -1: no more items
+        int job, g, win;       // win -1: the job does not fit 32-bit offsets, nothing is stored
+    };
+    const att_spmm_job *const jobs;
+    int64_t *const header;
+    int32_t *const err;
+    const int lane;
+    const uint32_t sbase;
+    const int n_items, n_jobs;
+    uint32_t xdst, idsrc;
+    int ch;
+    // drawn -> group range in flight -> rowptr in flight -> entered
+    int d_after;                                        // lane 0, in flight
+    int job, job_begin, job_end;                        // of the last item found
+    int r_job, r_g, r_fc, r_p0, r_p1;
+    int e_job, e_g, e_fc, e_start, e_end, e_pend, e_win;
+    Work f, p, pend;
+    int fid;
+    const int32_t *f_col;
+    const char *p_X;
+    const char *p_val;
+    int p_row_bytes;
+    unsigned n_x;
+    bool started;
+    bool p_whole, p_live;                               // p_live: the lane's piece lies inside F
+    uint32_t wbuf, rbuf;
+
+    __device__ __forceinline__ BatchStream(const att_spmm_job *jobs_, int64_t *header_, int32_t *err_, int lane_,
+                                           int warp, uint32_t sbase_)
+        : jobs(jobs_), header(header_), err(err_), lane(lane_), sbase(sbase_), n_items((int)header_[1]),
+          n_jobs((int)header_[0]) {
+        const int rg = lane / C::CPR;
+        ch = lane % C::CPR;
+        xdst = sbase + rg * C::RPL * C::XROW + ((ch ^ swz<C::XROW>(rg * C::RPL)) << 4);
+        idsrc = sbase + C::IDS + rg * C::RPL * 4;
+        job = -1;
+        job_begin = job_end = 0;
+        started = false;
+        find((int)blockIdx.x * C::NW + warp);
+        draw();
+        rows();
+        enter();
+        wbuf = rbuf = 0;
+        take();
+        copy();
+        pend = p;
+        wbuf = C::BUF;
+        __syncwarp();  // the copied chunk's ids have been read
+        take();
     }
-    const int n_items = (int)header[1];
-    unsigned int *const counter = reinterpret_cast<unsigned int *>(header + 4);
-    const int gid = lane >> 2, tig = lane & 3;
-    int pq = 0, cq = 0;
-
-    auto next_item = [&]() -> int {
-        unsigned int v = 0;
-        if (lane == 0) v = atomicAdd(counter, 1u);
-        v = __shfl_sync(0xffffffffu, v, 0);
-        return n_fixed + (int)v;
-    };
-
-    // producer cursor and the fields of its job it uses every step
-    int p_item = (int)blockIdx.x * kWarps + warp;
-    int p_step = 0, p_fc = 0, p_myc = -1;
-    PartInfo p_pi = {0, 0, 0};
-    const T *p_X = nullptr, *p_val = nullptr;  // p_val: the group's first value
-    const int32_t *p_col = nullptr;             // the group's first column id
-    int p_ldx = 0, p_nx = 0, p_F = 0;
-    // load item p_item (or the end marker) and hand it to the consumer
-    auto p_load = [&]() {
-        ring[warp][pq % kRing] = p_item;  // every lane writes the same value and reads its own
-        ++pq;
-        if (p_item >= n_items) return;
-        const att_spmm_job *pj = jobs + find_prefix(jobs, n_jobs, p_item, 0);
-        const int local = (int)(p_item - pj->item_begin);
-        p_F = (int)pj->F;
-        const int nch = (p_F + FC - 1) / FC;
-        const int g = local / nch;
-        p_fc = local - g * nch;
-        p_X = (const T *)pj->X;
-        p_ldx = (int)pj->ldx;
-        p_nx = (int)pj->n_x;
-        p_pi = group_info<WIDE>(pj->rowptr, __ldg(pj->group_part + g), __ldg(pj->group_part + g + 1),
-                                err);
-        p_val = (const T *)pj->val + p_pi.start * W;
-        p_col = pj->col + p_pi.start;
-        if (!job_small(pj)) {  // not addressed: one zero step, no store
-            if (err) atomicOr(err, 8);
-            p_pi.nreal = 0;
-            p_pi.nsteps = 1;
+    __device__ __forceinline__ void draw() {
+        if (lane == 0)
+            d_after = (int)gridDim.x * C::NW + (int)atomicAdd(reinterpret_cast<unsigned int *>(header + 4), 1u);
+    }
+    // item's job, group and feature chunk; the group's parts in flight
+    __device__ __forceinline__ void find(int item) {
+        r_fc = -1;
+        r_p0 = r_p1 = 0;
+        if (item >= n_items || item < 0) return;
+        while (item >= job_end) {
+            ++job;
+            job_begin = warp_uniform((int)jobs[job].item_begin);
+            job_end = job + 1 < n_jobs ? warp_uniform((int)jobs[job + 1].item_begin) : n_items;
         }
-        p_step = 0;
-    };
-    auto p_fetch = [&]() {
-        p_myc = -1;
-        if (p_item < n_items && p_step * 16 + (lane & 15) < p_pi.nreal)
-            p_myc = __ldg(p_col + p_step * 16 + (lane & 15));
-    };
-    auto issue = [&](int stage) {
-        const uint32_t xs = sbase + stage * C::STAGE;
-        const uint32_t vs = xs + C::XSTAGE;
-        const int c0 = p_step * 16;
-        int myc = p_myc;
-        // valid ids are -1 (padding) .. n_x - 1: checked once per id
-        if ((unsigned)(myc + 1) > (unsigned)p_nx) {
+        const int nch = warp_uniform(((int)jobs[job].F + FC - 1) / FC);
+        const int local = item - job_begin;
+        r_job = job;
+        r_g = nch == 1 ? local : local / nch;
+        r_fc = local - r_g * nch;
+        r_p0 = __ldg(jobs[job].group_part + r_g);
+        r_p1 = __ldg(jobs[job].group_part + r_g + 1);
+    }
+    __device__ __forceinline__ void rows() {
+        e_job = r_job;
+        e_g = r_g;
+        e_fc = r_fc;
+        e_start = e_end = e_pend = 0;
+        e_win = -1;
+        if (e_fc >= 0) {
+            const att_spmm_job *j = jobs + e_job;
+            e_start = __ldg(j->rowptr + 2 * r_p0);
+            e_end = __ldg(j->rowptr + 2 * r_p1 - 1);
+            e_pend = __ldg(j->rowptr + 2 * r_p1);
+            e_win = __ldg(j->window_of_part + r_p0);
+        }
+        const int nxt = warp_uniform(d_after);
+        draw();
+        find(nxt);
+    }
+    __device__ __forceinline__ void fetch_ids() { fid = lane < f.left ? __ldg(f_col + f.start + lane) : -1; }
+    __device__ __forceinline__ void enter() {
+        const PartInfo pi = part_check<8>(e_start, e_end, e_pend, err);
+        f.start = warp_uniform(pi.start);
+        f.left = warp_uniform(pi.nreal);
+        f.fc = e_fc;
+        f.job = e_job;
+        f.g = e_g;
+        f.win = warp_uniform(e_win);
+        if (f.fc >= 0) {
+            const att_spmm_job *j = jobs + f.job;
+            f_col = j->col;
+            if (!job_small(j)) {  // not addressed: nothing gathered, nothing stored
+                if (err) atomicOr(err, 8);
+                f.left = 0;
+                f.win = -1;
+            }
+        }
+        rows();
+        fetch_ids();
+    }
+    __device__ __forceinline__ void take() {
+        const bool same = p_is(f);
+        p = f;
+        if (p.fc < 0) return;
+        const att_spmm_job *j = jobs + p.job;
+        if (!same) {
+            const int F = (int)j->F, fe = p.fc * FC + ch * 8;
+            p_live = fe < F;
+            p_X = reinterpret_cast<const char *>(j->X) + 2 * (int64_t)fe;
+            p_val = reinterpret_cast<const char *>(j->val) + lane * 16;
+            p_row_bytes = 2 * (int)j->ldx;
+            n_x = (unsigned)j->n_x;
+        }
+        int c = fid;  // valid ids are -1 (padding) .. n_x - 1
+        const bool none = (unsigned)c >= n_x;
+        if (none && c != -1) {
             if (err) atomicOr(err, 1);
-            myc = -1;
+            c = -1;
         }
-        const int fbase = p_fc * FC;
-        const bool full = fbase + FC <= p_F;
+        p_whole = !__any_sync(0xffffffffu, none);
+        asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(sbase + C::IDS + 4 * lane), "r"(c) : "memory");
+        if (f.left > 32) {
+            f.start += 32;
+            f.left -= 32;
+            fetch_ids();
+        } else {
+            enter();
+        }
+        __syncwarp();
+    }
+    // the chunk continues the copy cursor's item
+    __device__ __forceinline__ bool p_is(const Work &w) {
+        const bool same = started && w.job == p.job && w.g == p.g && w.fc == p.fc;
+        started = true;
+        return same;
+    }
+    template <bool WHOLE>
+    __device__ __forceinline__ void copy_half(uint32_t dst, uint32_t ids) {
+        auto at = [&](int k) { return (dst ^ (swz<C::XROW>(k) << 4)) + k * C::XROW; };
+        int id[C::RPL];
+        lds_ids<C::RPL>(id, ids);
 #pragma unroll
-        for (int i = 0; i < 16 / C::RPP; ++i) {
-            const int r = i * C::RPP + lane / C::CPR;
-            const int ch = lane % C::CPR;
-            const int cidx = __shfl_sync(0xffffffffu, myc, r);
-            const int f = fbase + ch * 8;
-            const bool ok = cidx >= 0 && (full || f < p_F);
-            const int off = ok ? cidx * p_ldx + f : 0;
-            cp_async16(xs + r * C::XROW + ((ch ^ swz<C::XROW>(r)) << 4), p_X + off, ok ? 16 : 0);
+        for (int k = 0; k < C::RPL; ++k) {
+            const bool ok = WHOLE || id[k] >= 0;
+            cp_async16(at(k), p_X + (ok ? (int64_t)id[k] * p_row_bytes : 0), ok ? 16 : 0);
         }
-#pragma unroll
-        for (int q = lane; q < C::VCH; q += 32) {
-            const int e = q * 8;
-            const int blk = e / (W * WIDE);
-            const bool ok = c0 + blk * WIDE < p_pi.nreal;
-            const T *src = p_val + (c0 * W + e);
-            cp_async16(vs + q * 16, ok ? (const void *)src : (const void *)p_val, ok ? 16 : 0);
-        }
-    };
-    auto p_advance = [&]() {
-        if (++p_step >= p_pi.nsteps) {
-            p_item = next_item();
-            p_load();
-        }
-        p_fetch();
-    };
-
-    p_load();
-    p_fetch();
-#pragma unroll
-    for (int s = 0; s < S - 1; ++s) {
-        if (p_item < n_items) {
-            issue(s);
-            p_advance();
+    }
+    __device__ __forceinline__ void copy() {
+        if (p.fc >= 0 && p.left > 0) {
+            if (p_live) {  // pieces past F stay as they are (their products are never stored)
+                if (p_whole) {
+                    copy_half<true>(xdst + wbuf, idsrc);
+                    copy_half<true>(xdst + wbuf + C::HALF, idsrc + 64);
+                } else {
+                    copy_half<false>(xdst + wbuf, idsrc);
+                    if (p.left > 16) copy_half<false>(xdst + wbuf + C::HALF, idsrc + 64);
+                }
+            }
+            const bool ok = lane / 8 * 8 < p.left;  // a block past the group's real columns is zeros
+            cp_async16(sbase + C::VAL + wbuf + lane * 16, ok ? p_val + (int64_t)p.start * (W * 2) : p_val, ok ? 16 : 0);
         }
         cp_async_commit();
     }
+    __device__ __forceinline__ bool more() const { return pend.fc >= 0; }
+    __device__ __forceinline__ Work next() {
+        const Work c = pend;
+        copy();
+        pend = p;
+        __syncwarp();  // the copied chunk's ids have been read
+        take();
+        wbuf ^= C::BUF;
+        cp_async_wait<1>();
+        __syncwarp();
+        return c;
+    }
+    __device__ __forceinline__ void release() {
+        __syncwarp();
+        rbuf ^= C::BUF;
+    }
+};
 
-    float acc[C::MT][C::NT][4];
-#pragma unroll
-    for (int j = 0; j < C::MT; ++j)
-#pragma unroll
-        for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
+__global__ void __launch_bounds__(CfgBatch::NW * 32, 1)
+    k_spmm16_batched(const att_spmm_job *__restrict__ jobs, int64_t *__restrict__ header, int32_t *__restrict__ err) {
+    using C = CfgBatch;
+    constexpr int FC = 64, MT = FC / 16;
+    extern __shared__ __align__(128) unsigned char smem[];
+    const int lane = threadIdx.x & 31, warp = warp_uniform(threadIdx.x >> 5);
+    const uint32_t sbase = smem_u32(smem) + warp * C::WARP_SMEM;
+    // items, and the draws past them (three a warp), must be 32-bit
+    if (header[1] > (int64_t)INT32_MAX - 4 * (int64_t)gridDim.x * C::NW - 1) {
+        if (err && threadIdx.x == 0 && blockIdx.x == 0) atomicOr(err, 8);
+        return;
+    }
+    const int gid = lane >> 2, tig = lane & 3;
+    const int q = lane >> 3, rr = lane & 7;
+    const int xk = (q >> 1) * 8 + rr;
+    const uint32_t xlane = sbase + xk * C::XROW + (((q & 1) ^ swz<C::XROW>(xk)) << 4);
+    const uint32_t vlane = sbase + C::VAL + lane * 16;
 
-    int cstage = 0, pstage = S - 1;
-    for (;;) {
-        const int c_item = ring[warp][cq % kRing];
-        ++cq;
-        if (c_item >= n_items) break;
-        const att_spmm_job *cj = jobs + find_prefix(jobs, n_jobs, c_item, 0);
-        const int local = (int)(c_item - cj->item_begin);
-        const int F = (int)cj->F;
-        const int nch = (F + FC - 1) / FC;
-        const int g = local / nch;
-        const int fc = local - g * nch;
-        const int gp0 = __ldg(cj->group_part + g);
-        PartInfo pi = group_info<WIDE>(cj->rowptr, gp0, __ldg(cj->group_part + g + 1), nullptr);
-        const bool small = job_small(cj);
-        if (!small) pi.nsteps = 1;  // the producer streamed one zero step
-        for (int step = 0; step < pi.nsteps; ++step) {
-            cp_async_wait<S - 2>();
-            __syncwarp();
-            const uint32_t xs = sbase + cstage * C::STAGE;
-            const uint32_t vs = xs + C::XSTAGE;
-            uint32_t b[C::NT][2];
-            {
-                const int q = lane >> 3, rr = lane & 7;
-                if constexpr (C::NT == 2) {
-                    const int kb = q & 1, r = (q >> 1) * 8 + rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x4(vs + e * 2, b[0][0], b[0][1], b[1][0], b[1][1]);
-                } else {
-                    const int kb = q & 1, r = rr;
-                    const int e = (kb * 8 / WIDE) * W * WIDE + r * WIDE + (kb * 8) % WIDE;
-                    ldsm_x2(vs + e * 2, b[0][0], b[0][1]);
-                }
-            }
+    float acc[MT][1][4];
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const int q = lane >> 3, rr = lane & 7;
-                const int k = (q >> 1) * 8 + rr;
-                const int ch = 2 * j + (q & 1);
-                uint32_t a[4];
-                ldsm_x4_trans(xs + k * C::XROW + ((ch ^ swz<C::XROW>(k)) << 4), a[0], a[1], a[2],
-                              a[3]);
-#pragma unroll
-                for (int t = 0; t < C::NT; ++t) mma_16816<T>(acc[j][t], a, b[t][0], b[t][1]);
-            }
-            __syncwarp();
-            if (p_item < n_items) {
-                issue(pstage);
-                p_advance();
-            }
-            cp_async_commit();
-            cstage = cstage + 1 == S ? 0 : cstage + 1;
-            pstage = pstage + 1 == S ? 0 : pstage + 1;
+    for (int j = 0; j < MT; ++j) acc[j][0][0] = acc[j][0][1] = acc[j][0][2] = acc[j][0][3] = 0.f;
+
+    BatchStream st(jobs, header, err, lane, warp, sbase);
+    while (st.more()) {
+        const BatchStream::Work c = st.next();
+        if (c.left > 0) {
+            uint32_t b[2][1][2];
+            ldsm_x4(vlane + st.rbuf, b[0][0][0], b[0][0][1], b[1][0][0], b[1][0][1]);
+            half_mma<__half, 1, FC>(acc, xlane + st.rbuf, b[0]);
+            if (c.left > 16) half_mma<__half, 1, FC>(acc, xlane + st.rbuf + C::HALF, b[1]);
         }
-        const int wrow = __ldg(cj->window_of_part + gp0);
-        const int slot = __ldg(cj->group_slot + g);
-        const int f0 = fc * FC;
-        const bool full = f0 + FC <= F;
-        const int m_out = (int)cj->m_out;
-        // whole window: rows of Y; else rows of partial slot `slot` ([8, F], ld F)
-        float *const base = slot < 0 ? cj->Y + wrow * W * (int)cj->ldy : cj->partial + slot * W * F;
-        const int ld = slot < 0 ? (int)cj->ldy : F;
+        st.release();
+        if (c.left > 32) continue;
+        if (c.win >= 0) {
+            const att_spmm_job *cj = jobs + c.job;
+            const int slot = __ldg(cj->group_slot + c.g);
+            const int F = (int)cj->F, m_out = (int)cj->m_out, f0 = c.fc * FC + gid;
+            // whole window: rows of Y; else rows of partial slot `slot` ([8, F], ld F)
+            float *const base = slot < 0 ? cj->Y + c.win * 8 * (int)cj->ldy : cj->partial + slot * 8 * F;
+            const int ld = slot < 0 ? (int)cj->ldy : F;
 #pragma unroll
-        for (int t = 0; t < C::NT; ++t) {
-            const int rl0 = t * 8 + 2 * tig;
+            for (int h = 0; h < 2; ++h) {
+                const int rl = 2 * tig + h;
+                if (c.win * 8 + rl >= m_out) continue;
+                float *dst = base + rl * ld + f0;
 #pragma unroll
-            for (int j = 0; j < C::MT; ++j) {
-                const int fa = f0 + 16 * j + gid;
-#pragma unroll
-                for (int h = 0; h < 4; ++h) {
-                    const int rl = rl0 + (h & 1);
-                    const int f = fa + (h >> 1) * 8;
-                    if (small && rl < W && wrow * W + rl < m_out && (full || f < F))
-                        base[rl * ld + f] = acc[j][t][h];
-                    acc[j][t][h] = 0.f;
-                }
+                for (int j = 0; j < 2 * MT; ++j)
+                    if (f0 + 8 * j < F) dst[8 * j] = acc[j / 2][0][h + 2 * (j & 1)];
             }
         }
+#pragma unroll
+        for (int j = 0; j < MT; ++j) acc[j][0][0] = acc[j][0][1] = acc[j][0][2] = acc[j][0][3] = 0.f;
     }
     cp_async_wait<0>();
 }
@@ -2127,12 +2139,8 @@ extern "C" int att_host_device_pointer(const void *host, void **device) {
 }
 
 extern "C" size_t att_spmm_batched_grid(void) {
-    using C = CfgB<__half, 8, 64, 8, 3>;
-    auto kernel = k_spmm16_batched<8, 64, 8, 3>;
-    if (prepare(kernel, C::SMEM) != ATT_OK) return 0;
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kThreads, C::SMEM);
-    return (size_t)sm_count() * (per_sm > 0 ? per_sm : 1);
+    if (prepare(k_spmm16_batched, CfgBatch::SMEM) != ATT_OK) return 0;
+    return (size_t)sm_count();
 }
 
 extern "C" int att_spmm_batched(const att_spmm_job *jobs, int64_t *header, int64_t grid,
@@ -2141,18 +2149,14 @@ extern "C" int att_spmm_batched(const att_spmm_job *jobs, int64_t *header, int64
     ATT_CHECK(window == 8 && wide == 8, ATT_ERR_UNSUPPORTED,
               "the batched SpMM takes the (8-row, 8-wide) fp16 format");
     ATT_CHECK(jobs && header && grid > 0, ATT_ERR_INVALID, "null table or empty grid");
-    using C = CfgB<__half, 8, 64, 8, 3>;
-    auto kernel = k_spmm16_batched<8, 64, 8, 3>;
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
+    const int prep = KernelOf<k_spmm16_batched>::prepared(CfgBatch::SMEM);
     if (prep != ATT_OK) return prep;
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned side = (unsigned)(sm_count() * 8);
     k_zero_empty_batched<8><<<side, 256, 0, st>>>(jobs, header);
     int s = launch_status("k_zero_empty_batched");
     if (s != ATT_OK) return s;
-    kernel<<<(unsigned)grid, kThreads, C::SMEM, st>>>(jobs, header, err_flag);
+    k_spmm16_batched<<<(unsigned)grid, CfgBatch::NW * 32, CfgBatch::SMEM, st>>>(jobs, header, err_flag);
     s = launch_status("k_spmm16_batched");
     if (s != ATT_OK) return s;
     k_reduce_groups_batched<8><<<(unsigned)(sm_count() * 4), 256, 0, st>>>(jobs, header);

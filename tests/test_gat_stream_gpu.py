@@ -69,3 +69,27 @@ def test_runs(cuda, dt, F, wide, part, run, H, mode, slope):
                 got = (rmax[h].cpu().double() + torch.log(rsum[h].cpu().double()))[has]
                 assert (got - lse[has]).abs().max() <= 1e-4 * (1 + lse[has].abs().max())
                 assert torch.all(rsum[h].cpu()[~has] == 0)
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("F,H", [(32, 3), (64, 1), (64, 4), (128, 2)])
+def test_grad_prepare_forms(cuda, dt, F, H):
+    """The 16-byte form of the backward's first pass keeps the scalar form's
+    order of sums: the same bits (rows off the 16-byte grid take the latter)."""
+    from att_gb300 import _lib, ops
+    n = 1003
+    g = torch.Generator().manual_seed(F)
+    dout, out = (torch.rand(2, n, H * F, generator=g) * 2 - 1).cuda()
+    off = torch.empty(n * H * F + 1, device="cuda")[1:].view(n, H * F).copy_(dout)
+    got = []
+    for d in (dout, off):
+        hi, lo = torch.empty(2, n, H * F, dtype=dt, device="cuda")
+        c = torch.empty(H, n, device="cuda")
+        _lib.call("att_gat_grad_prepare", ops._p(d), H * F, ops._p(out), H * F, n, H, F, ops._p(hi), ops._p(lo),
+                  ops._DT[dt], H * F, ops._p(c), ops._stream())
+        got.append((hi, lo, c))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
+    ref = (dout.double() * out.double()).view(n, H, F).sum(2).t()
+    assert (got[0][2].double() - ref).abs().max() <= F * 2.0 ** -23
+    assert torch.equal(got[0][0], dout.to(dt))
