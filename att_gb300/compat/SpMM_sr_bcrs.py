@@ -16,7 +16,7 @@ from att_gb300 import ops
 
 
 def _check(t, name):
-    if not isinstance(t, torch.Tensor) or t.device.type != "cuda":
+    if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise TypeError("%s must be a CUDA tensor" % name)
 
 
@@ -29,7 +29,9 @@ def _forward(row_offsets, col_indices, values, t_window_row, t_atomic, rhs_matri
     if rhs_matrix.dtype != x_dtype:
         raise TypeError("rhs_matrix must be %s" % x_dtype)
     dimN, mOri = int(dimN), int(mOri)
-    X = rhs_matrix.reshape(-1, dimN)
+    X = rhs_matrix
+    if X.dim() != 2 or X.shape[1] != dimN:
+        X = X.reshape(-1, dimN)
     Fp = (dimN + granule - 1) // granule * granule
     if Fp != dimN:
         X = torch.nn.functional.pad(X, (0, Fp - dimN))

@@ -29,6 +29,10 @@ def _p(t):
 
 
 def _stream():
+    # the current stream's handle without building a Stream object (2.9 us a
+    # call, a fifth of a small SpMM's host time; 0.4 this way)
+    if torch.cuda.is_initialized():
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
     return torch.cuda.current_stream().cuda_stream
 
 
