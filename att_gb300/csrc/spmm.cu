@@ -940,7 +940,7 @@ __global__ void __launch_bounds__(kThreads) k_spmm_fp8(
 // stores them as float2.  This removes the shared-memory round trip of the
 // fp16 tile (4 KB of shared traffic and four 16-byte stores per lane per
 // step) and lets one work item cover 128 features.  2.45M nodes, F = 128:
-// 1.27 ms on the chunk stream, 1.77 ms in a per-step ring (bound by issue).
+// 1.30 ms on the chunk stream, 1.83 ms in a per-step ring (bound by issue).
 constexpr float kF8Shift = 32768.f;
 constexpr float kF8Unshift = 1.f / 32768.f;
 
@@ -1796,9 +1796,10 @@ constexpr int kTmaStages = 5;
 //  * spmm_gather: row-gather mechanism of the 16-bit kernel, 0 = cp.async
 //    (default), 1 = TMA tile::gather4, 2 = cp.async.bulk per row.
 //  * spmm_stages / spmm_fc: chunk buffers per warp of the 16-bit kernel (2, 3:
-//    two; 4: three) and features per work item for F > 64 (64 or 128).  169,343
-//    nodes, F = 128: 64 features x 2 buffers 78 us, x 3 83; 128 x 2 74, x 3 84;
-//    on the 2.45M-node graph 64 x 2 is the faster one.
+//    two; 4: three) and features per work item for F > 64 (64 or 128; until one
+//    of them is set, wide_items chooses).  Three buffers gain nothing: 2.45M
+//    nodes, F = 128, 64 features x 2 buffers 1,734 us, x 3 1,722; 128 x 2 1,549,
+//    x 3 1,613.
 //  * spmm_fp8: 1 = A fragments dequantized in registers (k_spmm_fp8r, 128
 //    features per item when F > 64), 0 = through an fp16 shared tile
 //    (k_spmm_fp8).
@@ -1806,7 +1807,8 @@ constexpr int kTmaStages = 5;
 enum SpmmOpt { kOptGather = 0, kOptStages, kOptFc, kOptFp8, kOptTf32, kNumOpts };
 const char *const kOptNames[kNumOpts] = {"spmm_gather", "spmm_stages", "spmm_fc", "spmm_fp8",
                                          "spmm_tf32"};
-std::atomic<int> g_opt[kNumOpts] = {{0}, {3}, {64}, {1}, {0}};
+constexpr int kFcByRule = 0;  // spmm_fc not set: reads as 64
+std::atomic<int> g_opt[kNumOpts] = {{0}, {3}, {kFcByRule}, {1}, {0}};
 thread_local int t_opt[kNumOpts] = {-1, -1, -1, -1, -1};
 
 inline int opt(SpmmOpt i) {
@@ -1881,6 +1883,28 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
     return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int64_t, false>>{});
 }
 
+// Features per work item of the 16-bit kernel where the caller has not chosen:
+// 128 when that leaves no more than half a 64-feature item unused in the last
+// item (an even number of 64-feature items) and there are parts for at least
+// two items per warp of the GPU (152 SMs x 12-13 warps); else 64.  The 128-wide
+// item reads a part's column list and values once for twice the features and
+// gathers twice the bytes per id.  Same additions in the same order, so the
+// results are the same.  us, 64 against 128 features per item, 8-row windows:
+//   parts        F = 72        96          128         136         192         256
+//   0.7K      12.2 12.3   12.1 12.3   11.6 11.4   12.9 14.8   12.2 14.2   13.1 13.1
+//   2.1K      17.2 17.4   16.7 17.5   15.9 16.0   18.8 24.1   18.2 22.5   20.6 21.1
+//   4.9K      34.9 30.3   30.8 28.8   28.8 27.2
+//   8.1K      32.4 29.9   31.2 29.3   29.0 28.4
+//   22K       85.4 72.3   78.8 67.7   71.9 66.8    112  148    103  121    130  119
+//   2.45M nodes           2100 1490   1734 1549                           3884 3363
+// and 16-row windows (300,000 nodes, degree 20) 309 246 at 96, 299 271 at 128.
+constexpr int64_t kWideItemParts = 4096;
+inline bool wide_items(int64_t F, int64_t n_parts) {
+    const int fc = opt(kOptFc);
+    if (fc != kFcByRule) return fc == 128;
+    return (F + 63) / 64 % 2 == 0 && n_parts >= kWideItemParts;
+}
+
 template <typename T, int W, int WIDE>
 int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, const int32_t *win,
                   const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
@@ -1900,14 +1924,14 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
         return launch16<T, W, 32, WIDE, 2>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
                                         m_out, ldy, err, st);
     if constexpr (W == 8 && WIDE == 8) {
-        if (opt(kOptGather) == 2 && (F <= 64 || opt(kOptFc) == 64))
+        if (opt(kOptGather) == 2 && (F <= 64 || opt(kOptFc) != 128))
             return launch16_bulk<T, 3>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
                                        m_out, ldy, err, st);
     }
 #define ATT_L16S(FCv, Sv)                                                                       \
     return launch16<T, W, FCv, WIDE, Sv>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, \
                                          Y, m_out, ldy, err, st)
-    if (F <= 64 || opt(kOptFc) == 64) {
+    if (F <= 64 || !wide_items(F, n_parts)) {
         if (opt(kOptStages) == 4) ATT_L16S(64, 3);
         ATT_L16S(64, 2);
     }
@@ -2074,6 +2098,7 @@ extern "C" int att_get_option(const char *key, int *value) {
     const int i = opt_index(key);
     ATT_CHECK(i >= 0, ATT_ERR_INVALID, "unknown option '%s'", key);
     *value = opt((SpmmOpt)i);
+    if (i == kOptFc && *value == kFcByRule) *value = 64;
     return ATT_OK;
 }
 

@@ -72,7 +72,9 @@ enum att_dtype {
  *                      8-wide blocks, 64-feature chunks).
  *   "spmm_stages": prefetch depth of the 16-bit cp.async kernel: 2 and 3 (the
  *                  default) two 32-column chunk buffers per warp, 4 three.
- *   "spmm_fc":     features per work item for F > 64 (64, the default, or 128).
+ *   "spmm_fc":     features per work item for F > 64: 64 or 128.  Until it is
+ *                  set it reads as 64, and calls with many parts whose F fills
+ *                  128-feature items take those (the results are the same).
  *   "spmm_fp8":    FP8 feature kernel: 1 = dequantized in registers (default),
  *                  0 = dequantized through an fp16 shared-memory tile.
  *   "spmm_tf32":   fp32-feature (3xTF32) kernel, features per item x chunk

@@ -114,3 +114,26 @@ def test_capture_replays(cuda):
     call()
     # parts of split windows add in any order
     assert torch.allclose(again, Y, rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("W", [8, 16])
+@pytest.mark.parametrize("F", [72, 96, 128, 136, 192, 256])
+@pytest.mark.parametrize("n_windows", [4095, 4096])
+def test_item_width_rule(cuda, W, F, n_windows):
+    """Either side of the part count from which wide features take 128-feature
+    items: the same bits as both widths asked for by name (unsplit windows, so
+    every output is one chain of additions), and the FP64 result."""
+    from att_gb300 import ops
+    n = n_windows * W
+    rng = np.random.default_rng(F)
+    rowptr = np.arange(0, 2 * n + 1, 2, dtype=np.int32)
+    col = np.sort(np.stack([rng.integers(0, n // 2, n), rng.integers(n // 2, n, n)], 1), 1).reshape(-1).astype(np.int32)
+    deg = np.full(n, 0.5, np.float16)
+    f = ops.block_convert(torch.from_numpy(rowptr), torch.from_numpy(col), torch.from_numpy(deg), window=W)
+    assert f.n_parts == n_windows
+    X = torch.from_numpy(rng.uniform(-1, 1, (n, F)).astype(np.float16))
+    got = [ops.spmm(f.rowptr, f.col, f.val, f.window_of_part, f.atomic, X.cuda(), n, window=W, shape=s).cpu()
+           for s in (None, ("spmm", 64, 3), ("spmm", 128, 3))]
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    ref = 0.25 * (X[col[0::2]].double() + X[col[1::2]].double())
+    assert torch.all((got[0].double() - ref).abs() <= 2 * 2.0 ** -24)
