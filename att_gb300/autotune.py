@@ -2,8 +2,8 @@
 
 Two shapes are tuned by measurement, not by a model:
 
-* ``att_spmm`` (one graph per call): features per work item and cp.async ring
-  depth of the 16-bit kernel (``spmm_fc`` x ``spmm_stages``) or of the fp32
+* ``att_spmm`` (one graph per call): features per work item and chunk
+  buffers of the 16-bit kernel (``spmm_fc`` x ``spmm_stages``) or of the fp32
   (3xTF32) kernel (``spmm_tf32``), or the FP8 dequantization kernel
   (``spmm_fp8``).  The best pair depends on how many
   warps stay resident against how deep each warp's prefetch is, which moves

@@ -50,15 +50,15 @@ FALLBACK_HBM_GBS = 6800.0
 # shape; otherwise it reports traffic null and an algorithmic fraction.
 MEASURED_TRAFFIC = {
     ("spmm_products_fp16", 1.0): {
-        "bytes": 9881965568 + 1404438784, "shape": ("spmm", 64, 3),
-        "kernel": "k_spmm16<__half, 8, 64, 8, 3, int, 1>", "ncu_ms": 2.128, "commit": "6b938d9",
-        "profile": "profiles/spmm16_products_fp16_full_dram.md",
-        "note": "read 9.88 GB + write 1.40 GB; X rows of hub columns hit L2 (37.0 % of sectors)"},
+        "bytes": 9795933696 + 1326489600, "shape": ("spmm", 128, 3),
+        "kernel": "k_spmm16<__half, 8, 128, 8, 2, int, 1>", "ncu_ms": 1.655, "commit": "e002ea2",
+        "profile": "profiles/chunk_stream_products_dram.md",
+        "note": "read 9.80 GB + write 1.33 GB; X rows of hub columns hit L2 (34.5 % of sectors)"},
     ("spmm_products_fp8", 1.0): {
-        "bytes": 5512719360 + 1383769344, "shape": ("fp8", 1),
-        "kernel": "k_spmm_fp8r<8, 128, 8, int, 1>", "ncu_ms": 1.805, "commit": "6b938d9",
-        "profile": "profiles/spmm_fp8r_products_fp8_full_dram.md",
-        "note": "read 5.51 GB + write 1.38 GB; L2 hit rate 48.7 % of sectors"},
+        "bytes": 5319319808 + 1289698048, "shape": ("fp8", 1),
+        "kernel": "k_spmm_fp8r<8, 128, 8, int, 1>", "ncu_ms": 1.280, "commit": "e002ea2",
+        "profile": "profiles/chunk_stream_products_dram.md",
+        "note": "read 5.32 GB + write 1.29 GB; L2 hit rate 44.0 % of sectors"},
 }
 METRIC = "SpMM/SDDMM HBM GB/s (% roofline); GAT step ms; serve p50/p99 vs plain"
 
