@@ -291,7 +291,10 @@ __global__ void __launch_bounds__((GCfg<T, F, MODE>::NW * 32), 1) k_gat_fused(co
                 for (int u = 0; u < 2; ++u) {
                     const float mn = fmaxf(m_run[u], mx[u]);
                     alpha[u] = mn == NEG_INF ? 1.f : __expf(m_run[u] - mn);
-                    l_run[u] *= alpha[u];
+                    // rounded here: contracted with the addition of the half
+                    // behind it, a row's sum would depend on which half of a
+                    // chunk moves its reference
+                    l_run[u] = __fmul_rn(l_run[u], alpha[u]);
                     m_run[u] = mn;
                     mref[u] = mn == NEG_INF ? 0.f : mn;
                 }

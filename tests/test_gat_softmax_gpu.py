@@ -1,0 +1,53 @@
+"""The online softmax of the fused GAT forward: its arithmetic does not depend
+on where a row's columns fall in the stream."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _graph(rows, n):
+    """CSR of {row: columns}, every other row empty."""
+    rowptr = torch.zeros(n + 1, dtype=torch.int32)
+    for r, c in rows.items():
+        rowptr[r + 1] = len(c)
+    col = torch.cat([torch.tensor(sorted(rows[r]), dtype=torch.int32) for r in sorted(rows)])
+    return torch.cumsum(rowptr, 0).to(torch.int32), col
+
+
+@pytest.mark.parametrize("dt", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("F", [32, 64, 128])
+@pytest.mark.parametrize("stats", [True, False])
+def test_reference_move_does_not_depend_on_the_half(cuda, dt, F, stats):
+    """Rows whose softmax reference moves between one group of 16 columns and
+    the next: once both groups are halves of one 32-column chunk, once the
+    second opens the next chunk (16 columns of another row stand before them).
+    The same operations on the same numbers: the same bits."""
+    from att_gb300 import gat
+    pairs = 40
+    n = 16 * pairs + 48
+    first, second = range(n - 32, n - 16), range(n - 16, n)  # the groups; the 16 columns before are `pre`
+    trigger = n - 1                                            # of row 0 alone: moves the whole window's references
+    g = torch.Generator().manual_seed(F)
+    rows = {}
+    for k in range(pairs):
+        for j in range(7):
+            cols = [c for c in list(first) + list(second)[:-1] if torch.rand(1, generator=g).item() < 0.7]
+            cols += [first[j], second[j]] + ([trigger] if j == 0 else [])
+            rows[16 * k + j] = rows[16 * k + 8 + j] = set(cols)
+        for j, c in enumerate(list(first) + list(second)[:-1]):  # every column is there in both windows
+            for w in (0, 8):
+                rows[16 * k + w + 1 + j % 6] = rows[16 * k + w + 1 + j % 6] | {c}
+        rows[16 * k + 8 + 7] = set(range(n - 48, n - 32))
+    G = gat.GATGraph(*_graph(rows, n))
+    s0 = torch.zeros(1, n)
+    s1 = torch.rand(1, n, generator=g) * 2 - 1
+    s1[0, list(second)] += 1.0
+    s1[0, trigger] = 12.0  # more than 8 above every other
+    X = (torch.rand(n, F, generator=g) * 2 - 1).to(dt)
+    out, rmax, rsum = G.attention(X.cuda(), mode=gat.MODE_ADD, s0=s0.cuda(), s1=s1.cuda(), stats=stats)
+    a = torch.arange(pairs)[:, None] * 16 + torch.arange(7)
+    for t in [out] + ([rmax[0], rsum[0]] if stats else []):
+        assert torch.equal(t[a].cpu(), t[a + 8].cpu())
+    if stats:
+        assert torch.all(rsum[0][a] > 0)
