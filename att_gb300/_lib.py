@@ -65,6 +65,10 @@ _SIGNATURES = {
                                         _c_i64, _c_i64, _c_i64, _c_vp, _c_int, _c_i64, _c_vp]),
     "att_rowsum": (_c_int, [_c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_int, _c_int, _c_vp, _c_int,
                             _c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_i64, _c_i64, _c_vp]),
+    "att_rowsum_scratch_bytes": (_c_sz, [_c_i64, _c_int, _c_i64]),
+    "att_rowsum_ordered": (_c_int, [_c_vp, _c_vp, _c_vp, _c_vp, _c_i64, _c_int, _c_int, _c_vp, _c_int,
+                                    _c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_i64, _c_i64, _c_vp, _c_sz,
+                                    _c_vp]),
     "att_map_to_quad": (_c_int, [_c_vp, _c_i64, _c_int, _c_int, _c_vp, _c_vp]),
     "att_slot_mask": (_c_int, [_c_vp, _c_i64, _c_vp, _c_i64, _c_vp]),
     "att_edge_softmax": (_c_int, [_c_vp, _c_i64, _c_vp, _c_i64, _c_i64, ctypes.c_float, _c_int,

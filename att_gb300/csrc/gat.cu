@@ -329,11 +329,12 @@ __global__ void __launch_bounds__(256) k_gather_slots_quad(const int32_t *__rest
     }
 }
 
-template <int HB>
-__global__ void __launch_bounds__(256) k_rowsum_slots_quad(
+// part_sums (ORDERED): where the sums of split windows' parts go, for k_rowsum_merge
+template <int HB, bool ORDERED>
+__global__ void __launch_bounds__(256, HB == 1 ? 8 : 5) k_rowsum_slots_quad(
     const int32_t *__restrict__ rowptr, const int32_t *__restrict__ map, const int32_t *__restrict__ win,
     const int32_t *__restrict__ atomic, int64_t n_parts, const void *vals, int vdt, int64_t vsh, int64_t vse,
-    int64_t H, float *out, int64_t osh, int64_t osm, int64_t m_out) {
+    int64_t H, float *out, int64_t osh, int64_t osm, int64_t m_out, float *__restrict__ part_sums) {
     const int lane = threadIdx.x & 31;
     const int64_t p = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (p >= n_parts) return;
@@ -360,11 +361,21 @@ __global__ void __launch_bounds__(256) k_rowsum_slots_quad(
         for (int k = 0; k < HB; ++k) {
             acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 2);
             acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], 1);
-            if ((lane & 3) == 0 && h0 + k < H && row >= 0 && row < m_out) {
-                float *dst = out + (h0 + k) * osh + row * osm;
-                if (add) red_add_f32(dst, acc[k]);
-                else *dst = acc[k];
-            }
+        }
+        if ((lane & 3) != 0) continue;
+        if (ORDERED && add) {
+            float *dst = part_sums + (p * H + h0) * 8 + (lane >> 2);
+#pragma unroll
+            for (int k = 0; k < HB; ++k)
+                if (h0 + k < H) dst[8 * k] = acc[k];
+        } else if (row >= 0 && row < m_out) {
+#pragma unroll
+            for (int k = 0; k < HB; ++k)
+                if (h0 + k < H) {
+                    float *dst = out + (h0 + k) * osh + row * osm;
+                    if (add) red_add_f32(dst, acc[k]);
+                    else *dst = acc[k];
+                }
         }
     }
 }
@@ -410,7 +421,7 @@ __global__ void k_rowsum_slots(const int32_t *__restrict__ rowptr, const int32_t
                                const int32_t *__restrict__ win, const int32_t *__restrict__ atomic,
                                int64_t n_parts, int wide, const void *vals, int vdt, int64_t vsh,
                                int64_t vse, int64_t H, float *out, int64_t osh, int64_t osm,
-                               int64_t m_out) {
+                               int64_t m_out, float *__restrict__ part_sums) {
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (wid >= n_parts * H) return;
@@ -440,10 +451,67 @@ __global__ void k_rowsum_slots(const int32_t *__restrict__ rowptr, const int32_t
         for (int r = 0; r < W; ++r)
             if (r == lane) v = acc[r];
         const int64_t row = row0 + lane;
-        if (row >= 0 && row < m_out) {
+        if (add && part_sums) {
+            part_sums[(p * H + h) * W + lane] = v;
+        } else if (row >= 0 && row < m_out) {
             float *dst = out + h * osh + row * osm;
             if (add) red_add_f32(dst, v);
             else *dst = v;
+        }
+    }
+}
+
+// The rows of split windows: the sums of a window's parts (consecutive, each at
+// part_sums[(part * H + h) * W + row]) added in part order with their
+// rounding errors kept beside the sum (Knuth's two-sum: as good as an fp64 sum,
+// whose additions run at a sixty-fourth of the fp32 rate here).  A warp
+// takes the split windows that open in its 32 parts, a lane per (head, row), so
+// a part's sums are read in one piece.
+// Adding them to the output with red.add instead let the order in which warps
+// ended decide the last bits, and a layer that rounds such a sum to 16 bits
+// showed it (a row of 21,000 terms; its gradients moved by up to 8e-5).
+// 169,343 nodes, 4 heads (1,114 split windows of up to 91 parts): the whole call 101 -> 108 us.
+template <int W>
+__global__ void __launch_bounds__(256) k_rowsum_merge(const int32_t *__restrict__ win,
+                                                      const int32_t *__restrict__ atomic, int64_t n_parts,
+                                                      const float *__restrict__ part_sums, int64_t H, float *out,
+                                                      int64_t osh, int64_t osm, int64_t m_out) {
+    const int lane = threadIdx.x & 31;
+    const int64_t p = (int64_t)blockIdx.x * 256 + threadIdx.x, p0 = p - lane;
+    int w = 0;
+    bool opens = false;
+    if (p < n_parts) {
+        w = win[p];
+        opens = atomic[p] != 0 && (p == 0 || win[p - 1] != w);
+    }
+    for (unsigned m = __ballot_sync(0xffffffffu, opens); m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        const int wq = __shfl_sync(0xffffffffu, w, l);
+        const int64_t per = H * W;  // outputs of a window
+        for (int64_t o0 = 0; o0 < per; o0 += 32) {
+            const int64_t o = o0 + lane;
+            float s = 0.f, err = 0.f;
+            for (int64_t k0 = p0 + l;; k0 += 32) {  // 32 parts at a time, up to the window's last
+                const bool in = k0 + lane < n_parts && win[k0 + lane] == wq;
+                const unsigned other = ~__ballot_sync(0xffffffffu, in);
+                const int n = other ? __ffs(other) - 1 : 32;
+                const float *src = part_sums + k0 * per + o;
+                for (int j = 0; j < n; j += 8) {  // eight loads in flight
+                    float v[8];
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) v[u] = o < per && j + u < n ? src[(j + u) * per] : 0.f;
+#pragma unroll
+                    for (int u = 0; u < 8; ++u) {
+                        const float t = s + v[u], b = t - s;
+                        err += (s - (t - b)) + (v[u] - b);
+                        s = t;
+                    }
+                }
+                if (n < 32) break;
+            }
+            const int64_t h = o / W, row = (int64_t)wq * W + (o - h * W);
+            // an infinite or NaN sum has no error term
+            if (o < per && row >= 0 && row < m_out) out[h * osh + row * osm] = isfinite(s) ? s + err : s;
         }
     }
 }
@@ -1029,17 +1097,14 @@ extern "C" int att_map_to_quad(const int32_t *map, int64_t n_slots, int window, 
     return launch_status("k_map_to_quad");
 }
 
-extern "C" int att_rowsum(const int32_t *rowptr, const int32_t *map,
-                          const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
-                          int window, int wide, const void *vals, int v_dtype,
-                          int64_t v_stride_h, int64_t v_stride_e, int64_t n_heads, float *out,
-                          int64_t out_stride_h, int64_t out_stride_n, int64_t m_out,
-                          void *stream) {
-    clear_error();
-    ATT_CHECK(window == 8 || window == 16, ATT_ERR_UNSUPPORTED, "window must be 8 or 16");
-    ATT_CHECK(wide > 0, ATT_ERR_INVALID, "bad wide");
-    cudaStream_t st = (cudaStream_t)stream;
-    if (m_out == 0 || n_heads == 0) return ATT_OK;
+namespace att {
+namespace {
+
+// part_sums: null, or [n_parts][n_heads][window] floats
+int rowsum(const int32_t *rowptr, const int32_t *map, const int32_t *window_of_part, const int32_t *atomic,
+           int64_t n_parts, int window, int wide, const void *vals, int v_dtype, int64_t v_stride_h,
+           int64_t v_stride_e, int64_t n_heads, float *out, int64_t out_stride_h, int64_t out_stride_n,
+           int64_t m_out, float *part_sums, cudaStream_t st) {
     ATT_CHECK(out != nullptr, ATT_ERR_INVALID, "null output");
     const int64_t n_w = (m_out + window - 1) / window;
     k_zero_rows_heads<<<(unsigned)((n_w + 255) / 256), 256, 0, st>>>(
@@ -1050,27 +1115,75 @@ extern "C" int att_rowsum(const int32_t *rowptr, const int32_t *map,
     if (warps == 0) return ATT_OK;
     ATT_CHECK(rowptr && map && window_of_part && atomic && vals, ATT_ERR_INVALID, "null pointer");
     if (window == 8 && wide == kQuad) {
-        const unsigned qgrid = (unsigned)((n_parts * 32 + 255) / 256);
-        if (n_heads == 1)
-            k_rowsum_slots_quad<1><<<qgrid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, vals, v_dtype,
-                                                          v_stride_h, v_stride_e, n_heads, out, out_stride_h,
-                                                          out_stride_n, m_out);
-        else
-            k_rowsum_slots_quad<4><<<qgrid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, vals, v_dtype,
-                                                          v_stride_h, v_stride_e, n_heads, out, out_stride_h,
-                                                          out_stride_n, m_out);
-        return launch_status("k_rowsum_slots_quad");
+        const unsigned grid = (unsigned)((n_parts * 32 + 255) / 256);
+        auto run = [&](auto kernel) {
+            kernel<<<grid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, vals, v_dtype, v_stride_h,
+                                         v_stride_e, n_heads, out, out_stride_h, out_stride_n, m_out, part_sums);
+        };
+        if (part_sums && n_heads == 1) run(k_rowsum_slots_quad<1, true>);
+        else if (part_sums) run(k_rowsum_slots_quad<4, true>);
+        else if (n_heads == 1) run(k_rowsum_slots_quad<1, false>);
+        else run(k_rowsum_slots_quad<4, false>);
+        s = launch_status("k_rowsum_slots_quad");
+    } else {
+        const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
+        auto run = [&](auto kernel) {
+            kernel<<<grid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, wide, vals, v_dtype,
+                                         v_stride_h, v_stride_e, n_heads, out, out_stride_h, out_stride_n, m_out,
+                                         part_sums);
+        };
+        if (window == 8) run(k_rowsum_slots<8>);
+        else run(k_rowsum_slots<16>);
+        s = launch_status("k_rowsum_slots");
     }
-    const unsigned grid = (unsigned)((warps * 32 + 255) / 256);
-    if (window == 8)
-        k_rowsum_slots<8><<<grid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts, wide,
-                                                vals, v_dtype, v_stride_h, v_stride_e, n_heads,
-                                                out, out_stride_h, out_stride_n, m_out);
-    else
-        k_rowsum_slots<16><<<grid, 256, 0, st>>>(rowptr, map, window_of_part, atomic, n_parts,
-                                                 wide, vals, v_dtype, v_stride_h, v_stride_e,
-                                                 n_heads, out, out_stride_h, out_stride_n, m_out);
-    return launch_status("k_rowsum_slots");
+    if (s != ATT_OK || !part_sums) return s;
+    const unsigned grid = (unsigned)((n_parts + 255) / 256);
+    auto merge = [&](auto kernel) {
+        kernel<<<grid, 256, 0, st>>>(window_of_part, atomic, n_parts, part_sums, n_heads, out, out_stride_h,
+                                             out_stride_n, m_out);
+    };
+    if (window == 8) merge(k_rowsum_merge<8>);
+    else merge(k_rowsum_merge<16>);
+    return launch_status("k_rowsum_merge");
+}
+
+}  // namespace
+}  // namespace att
+
+extern "C" int att_rowsum(const int32_t *rowptr, const int32_t *map,
+                          const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
+                          int window, int wide, const void *vals, int v_dtype,
+                          int64_t v_stride_h, int64_t v_stride_e, int64_t n_heads, float *out,
+                          int64_t out_stride_h, int64_t out_stride_n, int64_t m_out,
+                          void *stream) {
+    clear_error();
+    ATT_CHECK(window == 8 || window == 16, ATT_ERR_UNSUPPORTED, "window must be 8 or 16");
+    ATT_CHECK(wide > 0, ATT_ERR_INVALID, "bad wide");
+    if (m_out == 0 || n_heads == 0) return ATT_OK;
+    return rowsum(rowptr, map, window_of_part, atomic, n_parts, window, wide, vals, v_dtype, v_stride_h, v_stride_e,
+                  n_heads, out, out_stride_h, out_stride_n, m_out, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" size_t att_rowsum_scratch_bytes(int64_t n_parts, int window, int64_t n_heads) {
+    if (n_parts <= 0 || window <= 0 || n_heads <= 0) return 0;
+    return (size_t)n_parts * (size_t)window * (size_t)n_heads * sizeof(float);
+}
+
+extern "C" int att_rowsum_ordered(const int32_t *rowptr, const int32_t *map, const int32_t *window_of_part,
+                                  const int32_t *atomic, int64_t n_parts, int window, int wide, const void *vals,
+                                  int v_dtype, int64_t v_stride_h, int64_t v_stride_e, int64_t n_heads, float *out,
+                                  int64_t out_stride_h, int64_t out_stride_n, int64_t m_out, void *scratch,
+                                  size_t scratch_bytes, void *stream) {
+    clear_error();
+    ATT_CHECK(window == 8 || window == 16, ATT_ERR_UNSUPPORTED, "window must be 8 or 16");
+    ATT_CHECK(wide > 0, ATT_ERR_INVALID, "bad wide");
+    if (m_out == 0 || n_heads == 0) return ATT_OK;
+    const size_t need = att_rowsum_scratch_bytes(n_parts, window, n_heads);
+    ATT_CHECK(need == 0 || (scratch && ((uintptr_t)scratch & 3) == 0 && scratch_bytes >= need), ATT_ERR_WORKSPACE,
+              "scratch of %zu bytes, %zu needed (4-byte aligned)", scratch_bytes, need);
+    return rowsum(rowptr, map, window_of_part, atomic, n_parts, window, wide, vals, v_dtype, v_stride_h, v_stride_e,
+                  n_heads, out, out_stride_h, out_stride_n, m_out, need ? (float *)scratch : nullptr,
+                  (cudaStream_t)stream);
 }
 
 // ---------------------------------------------------------------------------

@@ -216,7 +216,10 @@ def rowsum(rowptr, qmap, win, atomic, window, vals, v_stride_h, v_stride_e, H, m
     else:
         out = torch.empty(m_out, H, 1, dtype=torch.float32, device=rowptr.device)
         osh, osn = out.stride(1), out.stride(0)
-    _lib.call("att_rowsum", _p(rowptr), _p(qmap), _p(win), _p(atomic), int(win.numel()), window,
+    # sums of the parts of split windows, added in a fixed order
+    n_parts = int(win.numel())
+    parts = torch.empty(n_parts * window * H, dtype=torch.float32, device=rowptr.device)
+    _lib.call("att_rowsum_ordered", _p(rowptr), _p(qmap), _p(win), _p(atomic), n_parts, window,
               QUAD, _p(vals), _DT[vals.dtype], v_stride_h, v_stride_e, H, _p(out), osh, osn,
-              m_out, _stream())
+              m_out, _p(parts), 4 * parts.numel(), _stream())
     return out

@@ -306,6 +306,16 @@ ATT_API int att_rowsum(const int32_t *rowptr, const int32_t *map,
                    int64_t v_stride_e, int64_t n_heads, float *out, int64_t out_stride_h,
                    int64_t out_stride_n, int64_t m_out, void *stream);
 
+/* The same sums with the parts of split windows added in part order, as
+ * exactly as in fp64 (att_rowsum adds them to `out` in the order in which they
+ * end): the same bits from run to run.  scratch: att_rowsum_scratch_bytes(...) bytes. */
+ATT_API size_t att_rowsum_scratch_bytes(int64_t n_parts, int window, int64_t n_heads);
+ATT_API int att_rowsum_ordered(const int32_t *rowptr, const int32_t *map, const int32_t *window_of_part,
+                   const int32_t *atomic, int64_t n_parts, int window, int wide, const void *vals,
+                   int v_dtype, int64_t v_stride_h, int64_t v_stride_e, int64_t n_heads, float *out,
+                   int64_t out_stride_h, int64_t out_stride_n, int64_t m_out, void *scratch,
+                   size_t scratch_bytes, void *stream);
+
 /* ======================================================================
  * Fused GAT attention layer (SDDMM -> LeakyReLU -> edge softmax -> SpMM in
  * one pass, no per-edge intermediates).  Replaces the reference's op chain of
