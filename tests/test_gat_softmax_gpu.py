@@ -1,5 +1,6 @@
 """The online softmax of the fused GAT forward: its arithmetic does not depend
-on where a row's columns fall in the stream."""
+on where a row's columns fall in the stream, and weights below the normal range
+of fp32 count."""
 import pytest
 import torch
 
@@ -51,3 +52,25 @@ def test_reference_move_does_not_depend_on_the_half(cuda, dt, F, stats):
         assert torch.equal(t[a].cpu(), t[a + 8].cpu())
     if stats:
         assert torch.all(rsum[0][a] > 0)
+
+
+@pytest.mark.parametrize("stats", [True, False])
+def test_weights_below_the_normal_range(cuda, stats):
+    """A weight e^-88 = 6.05e-39 is subnormal in fp32 and bf16 and still counts
+    where the features are large: sum = 1, out = e^-88 2^126 = 0.515.
+    Bound: bf16 rounds the weight to multiples of 2^-133; the argument of the
+    exponential (88 log2 e, rounded) is 4e-6 off, the weight 2^-149 / 6e-39."""
+    from att_gb300 import gat
+    tol = 2.0 ** -134 / 6.05e-39 + 1e-4
+    n = 64
+    G = gat.GATGraph(*_graph({r: {8 + r, 32 + r} for r in range(8)}, n))
+    X = torch.zeros(n, 32, dtype=torch.bfloat16)
+    X[32:40] = 2.0 ** 126
+    s1 = torch.zeros(1, n)
+    s1[0, 32:40] = -88.0
+    out, _, rsum = G.attention(X.cuda(), mode=gat.MODE_ADD, s0=torch.zeros(1, n).cuda(), s1=s1.cuda(), slope=1.0,
+                               stats=stats)
+    ref = 2.0 ** 126 * torch.exp(torch.tensor(-88.0, dtype=torch.float64)).item()
+    assert ((out[:8].cpu().double() - ref).abs() <= tol * ref).all()
+    if stats:
+        assert torch.all(rsum[0, :8] == 1)
