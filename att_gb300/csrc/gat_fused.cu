@@ -153,7 +153,8 @@ __global__ void __launch_bounds__((GCfg<T, F, MODE>::NW * 32), 1) k_gat_fused(co
     float m_run[2], mref[2], l_run[2];
     float acc[C::MT][4];
     bool first = true;
-    const bool convex = A.slope >= 0.f && A.slope <= 1.f;
+    // slope 0 is left out: there 0 * -inf is a NaN, which fmaxf would drop
+    const bool convex = A.slope > 0.f && A.slope <= 1.f;
 
     GatStream<C, T, IT> st(A.S, lane, warp, sbase, &queue);
     while (st.more()) {
@@ -255,7 +256,7 @@ __global__ void __launch_bounds__((GCfg<T, F, MODE>::NW * 32), 1) k_gat_fused(co
                     uint32_t w;
                     asm volatile("ld.shared.b32 %0, [%1];\n" : "=r"(w) : "r"(maddr[u] + st.rbuf + 16 * hf) : "memory");
                     const float x = sv[hf][u], y = A.slope * x;
-                    // the same value as x > 0 ? x : y where 0 <= slope <= 1
+                    // the same value as x > 0 ? x : y where 0 < slope <= 1
                     const float z = convex ? fmaxf(x, y) : x > 0.f ? x : y;
                     sv[hf][u] = (w & mbit[u]) ? z : NEG_INF;
                 }

@@ -1,6 +1,6 @@
 """The online softmax of the fused GAT forward: its arithmetic does not depend
-on where a row's columns fall in the stream, and weights below the normal range
-of fp32 count."""
+on where a row's columns fall in the stream, weights below the normal range
+of fp32 count, and infinite scores give what leaky_relu and softmax do."""
 import pytest
 import torch
 
@@ -74,3 +74,24 @@ def test_weights_below_the_normal_range(cuda, stats):
     assert ((out[:8].cpu().double() - ref).abs() <= tol * ref).all()
     if stats:
         assert torch.all(rsum[0, :8] == 1)
+
+
+@pytest.mark.parametrize("slope", [0.0, 0.2, 1.0, 1.5, -0.5])
+@pytest.mark.parametrize("value", [float("-inf"), float("inf"), float("nan")])
+def test_infinite_and_nan_scores(cuda, slope, value):
+    """A neighbour whose score is infinite or NaN, as leaky_relu and softmax have
+    it: with slope 0 a score of -inf is 0 * -inf, a NaN."""
+    from att_gb300 import gat
+    n = 64
+    G = gat.GATGraph(*_graph({r: {8 + r, 32 + r} for r in range(8)}, n))
+    X = torch.ones(n, 32, dtype=torch.float16)
+    s1 = torch.zeros(1, n)
+    s1[0, 32:36] = value
+    out, _, _ = G.attention(X.cuda(), mode=gat.MODE_ADD, s0=torch.zeros(1, n).cuda(), s1=s1.cuda(), slope=slope,
+                            stats=False)
+    e = torch.stack([s1[0, 8:16], s1[0, 32:40]], 1)
+    ref = torch.softmax(torch.where(e > 0, e, slope * e), 1).sum(1)  # features of 1: the weights' sum
+    got = out[:8].cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(ref)[:, None].expand_as(got))
+    ok = ~torch.isnan(ref)
+    assert ((got[ok] - 1).abs() <= 1e-5).all()
