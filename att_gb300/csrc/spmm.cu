@@ -21,9 +21,9 @@
 //    accuracy.
 //  * Output: a part of an unsplit window stores its whole W-row tile with
 //    plain stores; parts of split windows add with red.global.add.f32.  A
-//    small pre-pass, which the kernel behind it overlaps, zeroes only rows that
-//    no unsplit part writes (split windows, windows without parts, trailing
-//    rows), so Y needs no memset.
+//    small pre-pass, which the kernel behind it overlaps, zeroes a small Y whole
+//    and of a larger one only the rows that no unsplit part writes (split
+//    windows, windows without parts, trailing rows).
 #include "att_common.cuh"
 
 #include <cuda.h>
@@ -149,7 +149,7 @@ __global__ void __launch_bounds__((Cfg16<W, FC, WIDE, S>::NW * 32), 1)
         // ---- the part's last chunk: its W x FC tile ----
         const IT f0 = (IT)c.fc * FC + gid;
         const bool add = c.win & 1;
-        if (add) griddep_wait();  // the window's rows are zeroed by then
+        if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
@@ -661,7 +661,7 @@ __global__ void __launch_bounds__((CfgTF32<W, FC, WIDE, S>::NW * 32), 1)
         if (c.left > 32) continue;
         const IT f0 = (IT)c.fc * FC + 4 * gid;
         const bool add = c.win & 1;
-        if (add) griddep_wait();  // the window's rows are zeroed by then
+        if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
@@ -1076,7 +1076,7 @@ __global__ void __launch_bounds__((CfgF8R<W, FC, WIDE>::NW * 32), 1)
         // rows t * 8 + 2 tig (+1); F is a multiple of 16, so both features of
         // a pair are inside F together
         const bool add = c.win & 1;
-        if (add) griddep_wait();  // the window's rows are zeroed by then
+        if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
         const IT f0 = (IT)c.fc * FC + 2 * gid;
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
@@ -1620,6 +1620,27 @@ __global__ void k_zero_uncovered(const int32_t *__restrict__ win, const int32_t 
     }
 }
 
+// Y up to this size is zeroed whole, whatever the order of the windows (and of a
+// window's parts); the SpMM kernel then waits before its first store.
+// k_zero_uncovered takes larger ones and needs ascending windows.  It is the
+// cheaper of the two near the limit (65,536 nodes, degree 10, F = 128: 30 us a
+// call against 36; 16,384 nodes, F = 64: 20.8 against 19.2), but small part lists
+// in any order are calls that this function takes.
+constexpr int64_t kZeroAllBytes = 32ll << 20;
+inline bool zero_all(int64_t m_out, int64_t ldy) {
+    return m_out <= kZeroAllBytes / (int64_t)sizeof(float) / ldy;
+}
+
+__global__ void k_zero_all(float *__restrict__ Y, int64_t m_out, int64_t F, int64_t ldy, int vec) {
+    griddep_launch();
+    const int64_t per = vec ? F >> 2 : F;
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= m_out * per) return;
+    const int64_t r = t / per, f = t - r * per;
+    if (vec) *reinterpret_cast<float4 *>(Y + r * ldy + 4 * f) = make_float4(0.f, 0.f, 0.f, 0.f);
+    else Y[r * ldy + f] = 0.f;
+}
+
 template <typename K>
 int occupancy_grid(K kernel, int smem, int64_t items) {
     int per_sm = 0;
@@ -1686,7 +1707,7 @@ int launch16(const int32_t *rowptr, const int32_t *col, const void *val, const i
         const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, err};
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
         return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm16", A, Y, m_out, ldy);
     };
     if (small && F % FC == 0) return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int32_t, true>>{});
@@ -1734,7 +1755,7 @@ int launch_tf32(const int32_t *rowptr, const int32_t *col, const void *val, cons
         const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, err};
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
         return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_tf32", A, Y, m_out, ldy, vec_out);
     };
     if (small) return run(KernelOf<k_spmm_tf32<W, FC, WIDE, S, int32_t>>{});
@@ -1875,7 +1896,7 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
         const int prep = decltype(k)::prepared(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, err};
+        const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
         return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_fp8r", A, Y, m_out, ldy, vec_out);
     };
     if (small && F % FC == 0) return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int32_t, true>>{});
@@ -1985,9 +2006,15 @@ extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *v
     {
         const int64_t threads = (n_parts + 1) * 8;
         const int vec = F % 4 == 0 && ldy % 4 == 0 && ((uintptr_t)Y & 15) == 0;
-        k_zero_uncovered<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
-            window_of_part, atomic, n_parts, window, Y, m_out, F, ldy, vec);
-        s = launch_status("k_zero_uncovered");
+        if (zero_all(m_out, ldy)) {
+            const int64_t n = m_out * (vec ? F / 4 : F);
+            k_zero_all<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(Y, m_out, F, ldy, vec);
+            s = launch_status("k_zero_all");
+        } else {
+            k_zero_uncovered<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(
+                window_of_part, atomic, n_parts, window, Y, m_out, F, ldy, vec);
+            s = launch_status("k_zero_uncovered");
+        }
         if (s != ATT_OK) return s;
     }
     if (n_parts == 0) return ATT_OK;

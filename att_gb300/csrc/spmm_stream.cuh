@@ -129,6 +129,7 @@ struct StreamArgs {
     const float *xscale;  // EXTRA: per-row scales
     int64_t n_parts, n_x, F, ldx;
     int n_chunks;
+    int wait;  // every row was zeroed: no store before that is done
     int32_t *err;
 };
 
