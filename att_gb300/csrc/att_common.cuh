@@ -9,6 +9,7 @@
 #include <stdarg.h>
 
 #include "../../include/att_gb300.h"
+#include "per_device.cuh"
 
 namespace att {
 
@@ -46,6 +47,21 @@ inline int sm_count() {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
     return n > 0 ? n : 1;
+}
+
+// Opts kernel K in to `bytes` of dynamic shared memory, once per device (the
+// attribute belongs to the device that is current).  A kernel as a template
+// argument: instantiations that share a function type have flags of their own.
+template <auto K>
+int dynamic_smem(int bytes) {
+    static OncePerDevice once;
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return once.run(dev, [&] {
+        const cudaError_t e = cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+        if (e != cudaSuccess) cudaGetLastError();  // reported here, not by the next launch
+        return cuda_status(e, "cudaFuncSetAttribute");
+    });
 }
 
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

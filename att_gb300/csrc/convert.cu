@@ -41,7 +41,6 @@
 // All integer work; HBM- and L2-latency bound.
 #include "att_common.cuh"
 
-#include <mutex>
 
 namespace att {
 namespace {
@@ -1154,14 +1153,10 @@ int launch_unique_warp(unsigned grid, const int32_t *rowptr, const int32_t *col,
                        cudaStream_t st) {
     // register sort up to kWarpCap edges: no shared memory
     constexpr size_t smem = CAP <= kWarpCap ? 0 : (size_t)kWarpSortWarps * CAP * sizeof(KT);
-    auto kernel = k_unique_warp<KT, CAP, LO>;
+    constexpr auto kernel = k_unique_warp<KT, CAP, LO>;
     if (smem > 48 * 1024) {
-        static std::once_flag once;
-        static cudaError_t e = cudaSuccess;
-        std::call_once(once, [&] {
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        });
-        ATT_CUDA(e, "k_unique_warp shared memory");
+        const int prep = dynamic_smem<kernel>((int)smem);
+        if (prep != ATT_OK) return prep;
     }
     kernel<<<grid, kWarpSortWarps * 32, smem, st>>>(rowptr, col, nw, window, nnz, n_cols,
                                                     unsorted_only, ws);

@@ -21,7 +21,6 @@
 //   k_rowsum_slots    per-row sums of per-edge values through the map
 #include "att_common.cuh"
 
-#include <mutex>
 #include <type_traits>
 
 namespace att {
@@ -833,39 +832,28 @@ __global__ void __launch_bounds__(kSThreads) k_sddmm_tf32(SddmmArgs P) {
     }
 }
 
-template <typename K>
-int sddmm_launch(K kernel, int smem, int64_t items, const SddmmArgs &P, cudaStream_t st,
-                 std::once_flag &once, int &prep) {
-    std::call_once(once, [&] {
-        prep = cuda_status(
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-            "cudaFuncSetAttribute");
-    });
+template <auto K>
+int sddmm_launch(int smem, int64_t items, const SddmmArgs &P, cudaStream_t st) {
+    const int prep = dynamic_smem<K>(smem);
     if (prep != ATT_OK) return prep;
     if (items == 0) return ATT_OK;
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kSThreads, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K, kSThreads, smem);
     if (per_sm < 1) per_sm = 1;
     int64_t want = (items + kSWarps - 1) / kSWarps;
     int64_t cap = (int64_t)sm_count() * per_sm;
     int grid = (int)(want < cap ? want : cap);
-    kernel<<<grid, kSThreads, smem, st>>>(P);
+    K<<<grid, kSThreads, smem, st>>>(P);
     return launch_status("k_sddmm");
 }
 
 template <typename T, int W, int FC>
 int run_sddmm16(const SddmmArgs &P, cudaStream_t st) {
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    return sddmm_launch(k_sddmm16<T, W, FC>, SCfg<T, W, FC>::SMEM, P.n_parts * P.H, P, st, once,
-                        prep);
+    return sddmm_launch<k_sddmm16<T, W, FC>>(SCfg<T, W, FC>::SMEM, P.n_parts * P.H, P, st);
 }
 template <int W, int FC>
 int run_sddmm32(const SddmmArgs &P, cudaStream_t st) {
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    return sddmm_launch(k_sddmm_tf32<W, FC>, STf32<W, FC>::SMEM, P.n_parts * P.H, P, st,
-                        once, prep);
+    return sddmm_launch<k_sddmm_tf32<W, FC>>(STf32<W, FC>::SMEM, P.n_parts * P.H, P, st);
 }
 
 template <typename T, int W>

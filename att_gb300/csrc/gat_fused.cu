@@ -23,7 +23,6 @@
 // several chunks writes (m, l, acc) partials that k_gat_combine merges.
 #include "att_common.cuh"
 
-#include <mutex>
 #include <type_traits>
 
 namespace att {
@@ -521,17 +520,11 @@ __global__ void k_slot_mask(const int32_t *__restrict__ edge_slot, int64_t nnz, 
     if (s >= 0) atomicOr(mask + (s >> 5), 1u << (s & 31));
 }
 
-// Opts a kernel in to its dynamic shared memory, once per kernel
+// A kernel as a type, for the generic lambdas that launch one of two
 template <auto K>
-int gat_prepared(int smem) {
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    std::call_once(once, [&] {
-        prep = cuda_status(cudaFuncSetAttribute(K, cudaFuncAttributeMaxDynamicSharedMemorySize, smem),
-                           "cudaFuncSetAttribute");
-    });
-    return prep;
-}
+struct GatKernel {
+    static constexpr auto value = K;
+};
 
 template <typename T, int F, int MODE, bool PSPLIT>
 int run_gat(const GatArgs &P, cudaStream_t st, int64_t n_partial) {
@@ -546,15 +539,15 @@ int run_gat(const GatArgs &P, cudaStream_t st, int64_t n_partial) {
     const bool small = S.n_nodes * S.ld < lim && S.n_nodes * P.ldo < lim && S.H * S.n_nodes < lim &&
                        n_partial * S.H * kW * (F + 2) < lim;
     const int grid = (int)(items < sm_count() ? items : sm_count());
-    auto run = [&](auto prep, auto kernel) {
-        const int s = prep(C::SMEM);
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int s = dynamic_smem<kernel>(C::SMEM);
         if (s != ATT_OK) return s;
         kernel<<<grid, C::NW * 32, C::SMEM, st>>>(P);
         return launch_status("k_gat_fused");
     };
-    if (small)
-        return run(gat_prepared<k_gat_fused<T, F, MODE, PSPLIT, int32_t>>, k_gat_fused<T, F, MODE, PSPLIT, int32_t>);
-    return run(gat_prepared<k_gat_fused<T, F, MODE, PSPLIT, int64_t>>, k_gat_fused<T, F, MODE, PSPLIT, int64_t>);
+    if (small) return run(GatKernel<k_gat_fused<T, F, MODE, PSPLIT, int32_t>>{});
+    return run(GatKernel<k_gat_fused<T, F, MODE, PSPLIT, int64_t>>{});
 }
 
 template <typename T, int MODE>
@@ -883,14 +876,9 @@ int run_gat_bwd(const GatBwdArgs &P, cudaStream_t st) {
     using C = BCfg<T, F, SPLIT>;
     const int64_t items = P.n_parts * P.H;
     if (items == 0) return ATT_OK;
-    auto run = [&](auto kernel) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] {
-            prep = cuda_status(
-                cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM),
-                "cudaFuncSetAttribute");
-        });
+    auto run = [&](auto k) {
+        constexpr auto kernel = decltype(k)::value;
+        const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         int per_sm = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kGThreads, C::SMEM);
@@ -906,8 +894,8 @@ int run_gat_bwd(const GatBwdArgs &P, cudaStream_t st) {
     int64_t ld = P.ldx > P.ldd ? P.ldx : P.ldd;
     ld = ld > P.ldg ? ld : P.ldg;
     const bool small = P.n_nodes * ld < lim && P.n_nodes * P.H < lim && items < lim;
-    if (small) return run(k_gat_backward<T, F, SPLIT, int32_t>);
-    return run(k_gat_backward<T, F, SPLIT, int64_t>);
+    if (small) return run(GatKernel<k_gat_backward<T, F, SPLIT, int32_t>>{});
+    return run(GatKernel<k_gat_backward<T, F, SPLIT, int64_t>>{});
 }
 
 template <typename T>

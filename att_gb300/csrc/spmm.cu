@@ -1651,13 +1651,6 @@ int occupancy_grid(K kernel, int smem, int64_t items) {
     return (int)(want < cap ? (want > 0 ? want : 1) : cap);
 }
 
-template <typename K>
-int prepare(K kernel, int smem) {
-    // opt in to large dynamic shared memory once per kernel instantiation
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    return cuda_status(e, "cudaFuncSetAttribute");
-}
-
 // Launches a kernel that may start while the one before it on the stream (one
 // that calls griddep_launch) still runs; it calls griddep_wait before it
 // touches what that one writes.
@@ -1674,20 +1667,14 @@ int launch_dependent(void (*kernel)(P...), int grid, int threads, int smem, cuda
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cuda_status(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...), what);
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+    return launch_status(what);  // and clears the error: the next launch must not report it
 }
 
-// A kernel as a type: instantiations that share a function type still get their
-// own dynamic shared memory opt-in (the attribute is set once per kernel).
+// A kernel as a type, for the generic lambdas that launch one of several
 template <auto K>
 struct KernelOf {
     static constexpr auto value = K;
-    static int prepared(int smem) {
-        static std::once_flag once;
-        static int prep = ATT_OK;
-        std::call_once(once, [&] { prep = prepare(K, smem); });
-        return prep;
-    }
 };
 
 template <typename T, int W, int FC, int WIDE, int S>
@@ -1704,7 +1691,7 @@ int launch16(const int32_t *rowptr, const int32_t *col, const void *val, const i
     const bool small = ldx * (int64_t)sizeof(T) < lim && F < lim && items < lim;
     auto run = [&](auto k) {
         constexpr auto kernel = decltype(k)::value;
-        const int prep = decltype(k)::prepared(C::SMEM);
+        const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
         const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
@@ -1728,7 +1715,7 @@ int launch16_bulk(const int32_t *rowptr, const int32_t *col, const void *val, co
     const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
     auto run = [&](auto k) {
         constexpr auto kernel = decltype(k)::value;
-        const int prep = decltype(k)::prepared(SMEM);
+        const int prep = dynamic_smem<kernel>(SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = occupancy_grid(kernel, SMEM, items);
         kernel<<<grid, kThreads, SMEM, st>>>(rowptr, col, (const T *)val, win, atomic, n_parts,
@@ -1752,7 +1739,7 @@ int launch_tf32(const int32_t *rowptr, const int32_t *col, const void *val, cons
     const int vec_out = ldy % 4 == 0 && ((uintptr_t)Y & 15) == 0;
     auto run = [&](auto k) {
         constexpr auto kernel = decltype(k)::value;
-        const int prep = decltype(k)::prepared(C::SMEM);
+        const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
         const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
@@ -1781,10 +1768,8 @@ int launch16_tma(const int32_t *rowptr, const int32_t *col, const void *val, con
                  const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
                  int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, cudaStream_t st) {
     using C = CfgTma<W, FC, S>;
-    auto kernel = k_spmm16_tma<T, W, FC, WIDE, S>;
-    static std::once_flag once;
-    static int prep = ATT_OK;
-    std::call_once(once, [&] { prep = prepare(kernel, C::SMEM); });
+    constexpr auto kernel = k_spmm16_tma<T, W, FC, WIDE, S>;
+    const int prep = dynamic_smem<kernel>(C::SMEM);
     if (prep != ATT_OK) return prep;
     const int n_chunks = (int)((F + FC - 1) / FC);
     const int64_t items = n_parts * n_chunks;
@@ -1867,7 +1852,7 @@ int launch_fp8(const int32_t *rowptr, const int32_t *col, const void *val, const
     const bool small = n_x * ldx < lim && m_out * ldy < lim && items < lim;
     auto run = [&](auto k) {
         constexpr auto kernel = decltype(k)::value;
-        const int prep = decltype(k)::prepared(C::SMEM);
+        const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = occupancy_grid(kernel, C::SMEM, items);
         kernel<<<grid, kThreads, C::SMEM, st>>>(rowptr, col, (const __half *)val, win, atomic,
@@ -1893,7 +1878,7 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
     const int vec_out = (ldy % 2 == 0 && ((uintptr_t)Y & 7) == 0) ? 1 : 0;
     auto run = [&](auto k) {
         constexpr auto kernel = decltype(k)::value;
-        const int prep = decltype(k)::prepared(C::SMEM);
+        const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
         const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
@@ -2191,7 +2176,7 @@ extern "C" int att_host_device_pointer(const void *host, void **device) {
 }
 
 extern "C" size_t att_spmm_batched_grid(void) {
-    if (prepare(k_spmm16_batched, CfgBatch::SMEM) != ATT_OK) return 0;
+    if (dynamic_smem<k_spmm16_batched>(CfgBatch::SMEM) != ATT_OK) return 0;
     return (size_t)sm_count();
 }
 
@@ -2201,7 +2186,7 @@ extern "C" int att_spmm_batched(const att_spmm_job *jobs, int64_t *header, int64
     ATT_CHECK(window == 8 && wide == 8, ATT_ERR_UNSUPPORTED,
               "the batched SpMM takes the (8-row, 8-wide) fp16 format");
     ATT_CHECK(jobs && header && grid > 0, ATT_ERR_INVALID, "null table or empty grid");
-    const int prep = KernelOf<k_spmm16_batched>::prepared(CfgBatch::SMEM);
+    const int prep = dynamic_smem<k_spmm16_batched>(CfgBatch::SMEM);
     if (prep != ATT_OK) return prep;
     cudaStream_t st = (cudaStream_t)stream;
     const unsigned side = (unsigned)(sm_count() * 8);
