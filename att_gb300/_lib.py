@@ -26,6 +26,7 @@ _SIGNATURES = {
     "att_set_option": (_c_int, [ctypes.c_char_p, _c_int]),
     "att_set_thread_option": (_c_int, [ctypes.c_char_p, _c_int]),
     "att_get_option": (_c_int, [ctypes.c_char_p, ctypes.POINTER(_c_int)]),
+    "att_spmm_item_features": (_c_int, [_c_i64, _c_i64]),
     "att_block_workspace_bytes": (_c_sz, [_c_i64, _c_i64, _c_i64, _c_int]),
     "att_block_plan": (_c_int, [_c_vp, _c_vp, _c_i64, _c_i64, _c_i64, _c_int, _c_int, _c_int,
                                 _c_int, _c_vp, _c_sz, ctypes.POINTER(_c_i64),

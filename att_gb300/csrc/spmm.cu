@@ -1802,8 +1802,9 @@ constexpr int kTmaStages = 5;
 //  * spmm_gather: row-gather mechanism of the 16-bit kernel, 0 = cp.async
 //    (default), 1 = TMA tile::gather4, 2 = cp.async.bulk per row.
 //  * spmm_stages / spmm_fc: chunk buffers per warp of the 16-bit kernel (2, 3:
-//    two; 4: three) and features per work item for F > 64 (64 or 128; until one
-//    of them is set, wide_items chooses).  Three buffers gain nothing: 2.45M
+//    two; 4: three) and features per work item for F > 64 (a thread's 64 or 128 and
+//    a process-wide 128 are taken as they are; the process-wide 64, the default,
+//    leaves the choice to wide_items).  Three buffers gain nothing: 2.45M
 //    nodes, F = 128, 64 features x 2 buffers 1,734 us, x 3 1,722; 128 x 2 1,549,
 //    x 3 1,613.
 //  * spmm_fp8: 1 = A fragments dequantized in registers (k_spmm_fp8r, 128
@@ -1813,8 +1814,7 @@ constexpr int kTmaStages = 5;
 enum SpmmOpt { kOptGather = 0, kOptStages, kOptFc, kOptFp8, kOptTf32, kNumOpts };
 const char *const kOptNames[kNumOpts] = {"spmm_gather", "spmm_stages", "spmm_fc", "spmm_fp8",
                                          "spmm_tf32"};
-constexpr int kFcByRule = 0;  // spmm_fc not set: reads as 64
-std::atomic<int> g_opt[kNumOpts] = {{0}, {3}, {kFcByRule}, {1}, {0}};
+std::atomic<int> g_opt[kNumOpts] = {{0}, {3}, {64}, {1}, {0}};
 thread_local int t_opt[kNumOpts] = {-1, -1, -1, -1, -1};
 
 inline int opt(SpmmOpt i) {
@@ -1891,8 +1891,8 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
 
 // Features per work item of the 16-bit kernel where the caller has not chosen:
 // 128 when that leaves no more than half a 64-feature item unused in the last
-// item (an even number of 64-feature items) and there are parts for at least
-// two items per warp of the GPU (152 SMs x 12-13 warps); else 64.  The 128-wide
+// item (an even number of 64-feature items) and there are at least 4096 parts
+// (two items for each of the 152 x 12 warps that take them); else 64.  The 128-wide
 // item reads a part's column list and values once for twice the features and
 // gathers twice the bytes per id.  Same additions in the same order, so the
 // results are the same.  us, 64 against 128 features per item, 8-row windows:
@@ -1906,9 +1906,12 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
 // and 16-row windows (300,000 nodes, degree 20) 309 246 at 96, 299 271 at 128.
 constexpr int64_t kWideItemParts = 4096;
 inline bool wide_items(int64_t F, int64_t n_parts) {
-    const int fc = opt(kOptFc);
-    if (fc != kFcByRule) return fc == 128;
+    if (t_opt[kOptFc] >= 0) return t_opt[kOptFc] == 128;
+    if (g_opt[kOptFc].load(std::memory_order_relaxed) == 128) return true;
     return (F + 63) / 64 % 2 == 0 && n_parts >= kWideItemParts;
+}
+inline int item_features(int64_t F, int64_t n_parts) {
+    return F <= 32 ? 32 : F <= 64 || !wide_items(F, n_parts) ? 64 : 128;
 }
 
 template <typename T, int W, int WIDE>
@@ -1937,7 +1940,7 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
 #define ATT_L16S(FCv, Sv)                                                                       \
     return launch16<T, W, FCv, WIDE, Sv>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, \
                                          Y, m_out, ldy, err, st)
-    if (F <= 64 || !wide_items(F, n_parts)) {
+    if (item_features(F, n_parts) == 64) {
         if (opt(kOptStages) == 4) ATT_L16S(64, 3);
         ATT_L16S(64, 2);
     }
@@ -2110,9 +2113,10 @@ extern "C" int att_get_option(const char *key, int *value) {
     const int i = opt_index(key);
     ATT_CHECK(i >= 0, ATT_ERR_INVALID, "unknown option '%s'", key);
     *value = opt((SpmmOpt)i);
-    if (i == kOptFc && *value == kFcByRule) *value = 64;
     return ATT_OK;
 }
+
+extern "C" int att_spmm_item_features(int64_t F, int64_t n_parts) { return item_features(F, n_parts); }
 
 extern "C" size_t att_spmm_groups_scratch_bytes(int64_t n_parts, int64_t n_windows) {
     if (n_parts < 0) n_parts = 0;

@@ -72,9 +72,10 @@ enum att_dtype {
  *                      8-wide blocks, 64-feature chunks).
  *   "spmm_stages": prefetch depth of the 16-bit cp.async kernel: 2 and 3 (the
  *                  default) two 32-column chunk buffers per warp, 4 three.
- *   "spmm_fc":     features per work item for F > 64: 64 or 128.  Until it is
- *                  set it reads as 64, and calls with many parts whose F fills
- *                  128-feature items take those (the results are the same).
+ *   "spmm_fc":     features per work item for F > 64: 64 or 128.  The
+ *                  process-wide 64 (the default) lets calls with many parts
+ *                  whose F fills 128-feature items take those (the results are
+ *                  the same); a thread's 64 is 64.
  *   "spmm_fp8":    FP8 feature kernel: 1 = dequantized in registers (default),
  *                  0 = dequantized through an fp16 shared-memory tile.
  *   "spmm_tf32":   fp32-feature (3xTF32) kernel, features per item x chunk
@@ -82,6 +83,9 @@ enum att_dtype {
 ATT_API int att_set_option(const char *key, int value);
 ATT_API int att_set_thread_option(const char *key, int value);
 ATT_API int att_get_option(const char *key, int *value);
+/* Features per work item that a 16-bit att_spmm call of the calling thread takes
+ * with cp.async row gathers (32, 64 or 128). */
+ATT_API int att_spmm_item_features(int64_t F, int64_t n_parts);
 
 /* Human-readable name of a status. */
 ATT_API const char *att_status_string(int status);
