@@ -92,6 +92,18 @@ def spmm_candidates(x_dtype, F):
     return []
 
 
+def canonical_shape(c):
+    """The first of the launch shapes that run the same kernel as `c`: two of
+    the 16-bit kernel's prefetch depths (2, 3) and two of the fp32 kernel's
+    shapes (0, 3) are one instantiation each."""
+    if c is None:
+        return None
+    c = tuple(c)
+    if c[0] == "spmm" and c[2] == 3:
+        return ("spmm", c[1], 2)
+    return ("tf32", 0) if c == ("tf32", 3) else c
+
+
 def apply_shape(c):
     """Set the calling thread's att_spmm launch shape to candidate `c`."""
     ops.set_launch_shape(c)
@@ -100,7 +112,8 @@ def apply_shape(c):
 def tune_spmm(fmt, X, m_out, x_scale=None, out=None, val=None, tuner=None):
     """Time att_spmm's launch shapes on this format and features (block
     values `val`, default the format's own) and return (choice, {choice:
-    ms}).  Candidates are applied to the calling thread only and the thread
+    ms}); shapes that run the same kernel are timed once and share its time.
+    Candidates are applied to the calling thread only and the thread
     is returned to the defaults afterwards: pass the choice to
     ``ops.spmm(..., shape=choice)`` for the calls it was tuned for.  Shapes
     with nothing to tune (fp32 features with F <= 32) return (None, {})."""
@@ -124,9 +137,10 @@ def tune_spmm(fmt, X, m_out, x_scale=None, out=None, val=None, tuner=None):
         ops.spmm(fmt.rowptr, fmt.col, vals, fmt.window_of_part, fmt.atomic, X, m_out,
                  window=fmt.window, wide=fmt.wide, out=Y, x_scale=x_scale, shape=cur[0])
     try:
-        return tuner.best(key, cands, setup, run)
+        choice, table = tuner.best(key, [c for c in cands if canonical_shape(c) == c], setup, run)
     finally:
         clear_shape()
+    return choice, {c: table[canonical_shape(c)] for c in cands}
 
 
 def tune_group_parts(requests, candidates=(1, 2, 4, 8), tuner=None):

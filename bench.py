@@ -1283,9 +1283,10 @@ def roofline(wl, avg_launch_ms, shape):
     kbytes = getattr(wl, "bytes_fused", wl.bytes_alg)
     alg = kbytes / t / 1e9
     mt = MEASURED_TRAFFIC.get((wl.name, 1.0 if getattr(wl, "scale", 1.0) == 1.0 else wl.scale))
-    if mt is not None and mt.get("shape") is not None and shape is not None \
-            and tuple(mt["shape"]) != tuple(shape):
-        mt = None  # captured on another launch shape: its bytes are not this kernel's
+    if mt is not None and mt.get("shape") is not None and shape is not None:
+        from att_gb300.autotune import canonical_shape
+        if canonical_shape(mt["shape"]) != canonical_shape(shape):
+            mt = None  # captured on another launch shape: its bytes are not this kernel's
     comp = getattr(wl, "bytes_compulsory", None)
     roof = {"bound": "hbm", "peak": peak, "unit": "GB/s", "peak_kind": peak_kind,
             "kernel": getattr(wl, "kernel_name", "att_spmm (k_zero_uncovered + k_spmm16)"),
