@@ -21,13 +21,21 @@ from .ops import _DT, _p, _stream, require_cuda
 QUAD = 4
 
 
+def _quad_kernel_takes(m, window, wide):
+    """Whether att_map_to_quad takes this map: a flat int32 one on the current
+    device (the kernel runs on that device's stream), contiguous, 16-byte aligned,
+    of whole blocks of whole quads."""
+    return (m.is_cuda and m.device.index == torch.cuda.current_device() and m.dtype == torch.int32
+            and m.dim() == 1 and m.is_contiguous() and wide % QUAD == 0
+            and m.numel() % (window * wide) == 0 and m.data_ptr() % 16 == 0)
+
+
 def map_to_quad(map_std, window, wide):
     """Permute a slot map from the block-width-``wide`` layout to the quad layout."""
     if wide == QUAD or map_std is None or map_std.numel() == 0:
         return map_std
     n = map_std.numel()
-    if (map_std.is_cuda and map_std.dtype == torch.int32 and map_std.is_contiguous() and wide % QUAD == 0
-            and n % (window * wide) == 0 and map_std.data_ptr() % 16 == 0):
+    if _quad_kernel_takes(map_std, window, wide):
         out = torch.empty_like(map_std)
         _lib.call("att_map_to_quad", _p(map_std), n, window, wide, _p(out), _stream())
         return out
