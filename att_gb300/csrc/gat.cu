@@ -1053,8 +1053,9 @@ extern "C" int att_gather_slot_values(const int32_t *map, int64_t n_slots, int w
             if (out_dtype == ATT_BF16) return run((__nv_bfloat16 *)out, std::integral_constant<int, 8>{}, v);
             return run((float *)out, std::integral_constant<int, 4>{}, v);
         };
-        const bool fits = out_dtype == ATT_F32 ? out_wide == 4 && out_stride_h % 4 == 0
-                                               : out_wide == 8 && out_stride_h % 8 == 0;
+        const bool out16 = out_dtype == ATT_F16 || out_dtype == ATT_BF16;
+        const bool fits = out16 ? out_wide == 8 && out_stride_h % 8 == 0
+                                : out_wide == 4 && out_stride_h % 4 == 0;
         if (fits && (n_slots >> 2) < ((int64_t)1 << 38)) {
             if (v_dtype == ATT_F16) return with((__half *)nullptr);
             if (v_dtype == ATT_BF16) return with((__nv_bfloat16 *)nullptr);
