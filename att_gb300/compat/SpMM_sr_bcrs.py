@@ -30,7 +30,7 @@ def _forward(row_offsets, col_indices, values, t_window_row, t_atomic, rhs_matri
         raise TypeError("rhs_matrix must be %s" % x_dtype)
     dimN, mOri = int(dimN), int(mOri)
     X = rhs_matrix
-    if X.dim() != 2 or X.shape[1] != dimN:
+    if X.dim() != 2 or X.shape[1] != dimN or dimN == 0:  # reshape refuses a width of 0
         X = X.reshape(-1, dimN)
     Fp = (dimN + granule - 1) // granule * granule
     if Fp != dimN:
