@@ -385,7 +385,7 @@ __global__ void __launch_bounds__((GCfg<T, F, MODE>::NW * 32), 1) k_gat_fused(co
             if (c.left > 16) aggregate(sv[1], 1);
         }
         st.release();
-        first = c.left <= 32;
+        first = c.left <= 32 && c.slot != kGoesOn;
         if (!first || c.win < 0) continue;
         // row sums: the lanes' partial sums over their own columns
 #pragma unroll

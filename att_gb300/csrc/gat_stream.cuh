@@ -64,8 +64,9 @@ struct GChunk {
     int start, left;  // first condensed column, real columns left in the run
     int h;            // head, -1: no more items
     int win;          // window, -1: an empty run (nothing to write)
-    int slot;         // run_slot
+    int slot;         // run_slot, or kGoesOn: more of the run follows its last chunk
 };
+constexpr int kGoesOn = -2;
 
 // IT: index type of items and element offsets (int32_t when every offset fits)
 template <typename C, typename T, typename IT>
@@ -133,6 +134,15 @@ struct GatStream {
             }
         }
     }
+    struct Part {
+        int start, end, pend;
+        bool good;  // starts and ends on a block boundary
+    };
+    __device__ __forceinline__ Part part(int k) const {
+        const int s = __ldg(A.rowptr + 2 * (int64_t)k), e = __ldg(A.rowptr + 2 * (int64_t)k + 1),
+                  q = __ldg(A.rowptr + 2 * (int64_t)k + 2);
+        return {s, e, q, (s & (A.wide - 1)) == 0 && (q & (A.wide - 1)) == 0 && q >= e};
+    }
     // its rowptr; the next drawn item's range
     __device__ __forceinline__ void rows() {
         e_item = r_item;
@@ -147,11 +157,8 @@ struct GatStream {
             e_pend = __ldg(A.rowptr + 2 * (int64_t)e_p1);
             e_win = __ldg(A.win + e_p0);
             // every part of the run starts and ends on a block boundary
-            for (int k = e_p0 + lane; k < e_p1; k += 32) {
-                const int s = __ldg(A.rowptr + 2 * (int64_t)k), e = __ldg(A.rowptr + 2 * (int64_t)k + 1),
-                          q = __ldg(A.rowptr + 2 * (int64_t)k + 2);
-                if ((s & (A.wide - 1)) != 0 || (q & (A.wide - 1)) != 0 || q < e) e_end = INT32_MIN;
-            }
+            for (int k = e_p0 + lane; k < e_p1; k += 32)
+                if (!part(k).good) e_end = INT32_MIN;
         }
         e_near = false;
         const int nxt = warp_uniform(d_after);
@@ -169,17 +176,34 @@ struct GatStream {
     }
     __device__ __forceinline__ void fetch_ids() { fid = lane < f.left ? __ldg(A.col + f.start + lane) : -1; }
     __device__ __forceinline__ void enter() {
-        const bool bad = __any_sync(0xffffffffu, e_end == INT32_MIN);
-        if (bad && A.err) atomicOr(A.err, 2);
         f.start = warp_uniform(e_start);
-        f.left = warp_uniform(bad || e_end <= e_start ? 0 : e_end - e_start);
+        f.left = warp_uniform(e_end <= e_start ? 0 : e_end - e_start);
         f_pend = warp_uniform(e_pend - e_start);
         f.win = warp_uniform(e_win);
         f.slot = warp_uniform(e_slot);
         const int item = warp_uniform(e_item);
         f.h = item < n_items ? (H == 1 ? 0 : item - item / H * H) : -1;
-        rows();
+        // a run with a misaligned part among its parts goes one good part at a time
+        if (__any_sync(0xffffffffu, e_end == INT32_MIN)) good_part();
+        if (f.slot != kGoesOn) rows();
         fetch_ids();
+    }
+    // The next good part of the run; the run's other ones, if any, by later calls.
+    __device__ __forceinline__ void good_part() {
+        if (A.err) atomicOr(A.err, 2);
+        f.left = f_pend = 0;
+        for (int k = e_p0; k < e_p1; ++k) {
+            const Part t = part(k);
+            if (!t.good || t.end <= t.start) continue;
+            if (f.left > 0) {
+                e_p0 = k;
+                f.slot = kGoesOn;
+                break;
+            }
+            f.start = warp_uniform(t.start);
+            f.left = warp_uniform(t.end - t.start);
+            f_pend = warp_uniform(t.pend - t.start);
+        }
     }
     __device__ __forceinline__ void take() {
         p = f;
