@@ -86,7 +86,7 @@ namespace att {
 namespace {
 
 struct GatArgs {
-    GStreamArgs S;                // tile 0: X' rows; scalar 0: s1 (mode 1)
+    GStreamArgs S;                // rows: X'; scalar: s1 (mode 1)
     const float *s0;              // [H][n_nodes] row scores (mode 1)
     float slope;
     float *out;                   // [n_nodes, H*F] rows of ldo
@@ -98,8 +98,8 @@ struct GatArgs {
 // Warps per SM: 16 leave 128 registers a thread; fp32 X' is bounded by shared
 // memory (12 at 64 features).
 template <typename T, int F, int MODE>
-struct GCfg : GStreamCfg<F * (int)sizeof(T), 1, MODE == 1 ? 1 : 0, false, sizeof(T) == 4 ? 32 * kW * 4 : 0,
-                         2, F == 128 ? 12 : 16> {
+struct GCfg : GStreamCfg<F * (int)sizeof(T), MODE == 1, sizeof(T) == 4 ? 32 * kW * 4 : 0, 2,
+                         F == 128 ? 12 : 16> {
     static constexpr bool F32 = sizeof(T) == 4;  // fp32 X': 3xTF32 products
     static constexpr int MT = F / 16;
 };
@@ -118,7 +118,7 @@ __global__ void __launch_bounds__((GCfg<T, F, MODE>::NW * 32), 1) k_gat_fused(co
     const unsigned char *sgen = smem + warp * C::WARP_SMEM;
     const int gid = lane >> 2, tig = lane & 3;
     const IT H = (IT)A.S.H, n_nodes = (IT)A.S.n_nodes, ldx = (IT)A.S.ld, ldo = (IT)A.ldo;
-    const T *X = (const T *)A.S.X[0];
+    const T *X = (const T *)A.S.X;
     const float NEG_INF = -INFINITY;
     // logits may exceed a row's reference by this much before it moves
     constexpr float kLazy = 8.f;
@@ -966,7 +966,7 @@ extern "C" int att_gat_forward(const int32_t *rowptr, const int32_t *col, const 
     ATT_CHECK(n_multi == 0 || (partial && multi_chunk_begin), ATT_ERR_INVALID,
               "split windows need the partial buffer");
     GatArgs P{GStreamArgs{rowptr, col, window_of_part, slot_mask, chunk_begin, chunk_slot, n_chunks, n_heads, n_nodes,
-                          F, wide, {Xp, nullptr}, ldx, {s1, nullptr, nullptr, nullptr}, err_flag},
+                          F, wide, Xp, ldx, s1, err_flag},
               s0, slope, out, ldo, row_max, row_sum, partial};
     int s;
     // partial slots are at most one per chunk

@@ -2,7 +2,7 @@
 // stream of the SpMM kernels (spmm_stream.cuh: 32 condensed columns at a time,
 // three cursors a chunk apart, one CTA per SM whose warps draw their items from
 // a counter) over work items (run of parts of one window, head), with the
-// occupancy bits of the chunk's slots and per-column scalars beside the rows.
+// occupancy bits of the chunk's slots and a per-column scalar beside the rows.
 // Included by gat_fused.cu.
 //
 // The kernels are bound by issue and latency (X' fits L2): the ring with a
@@ -22,20 +22,18 @@ __device__ __forceinline__ int swz_rb(int r) {
     else return (r >> 1) & 3;
 }
 
-// A warp's shared memory: S chunk buffers (TILES tiles of 32 rows of XROW bytes,
-// 32 bytes of occupancy bits, NS x 32 scalars, 32 column ids if IDSOUT), the
-// copied chunk's ids, TAIL bytes of the kernel's own.
-template <int XROW_, int TILES_, int NS_, bool IDSOUT_, int TAIL_, int S_, int MAXW>
+// A warp's shared memory: S chunk buffers (32 rows of XROW bytes, 32 bytes of
+// occupancy bits in 128, 32 scalars if SCALAR), the copied chunk's ids, TAIL bytes
+// of the kernel's own.
+template <int XROW_, bool SCALAR_, int TAIL_, int S_, int MAXW>
 struct GStreamCfg {
-    static constexpr int XROW = XROW_, TILES = TILES_, NS = NS_;
-    static constexpr bool IDSOUT = IDSOUT_;
+    static constexpr int XROW = XROW_;
+    static constexpr bool SCALAR = SCALAR_;
     static constexpr int S = S_;
     static constexpr int HALF = 16 * XROW;
-    static constexpr int TILE = 2 * HALF;
-    static constexpr int MASK = TILES * TILE;
+    static constexpr int MASK = 2 * HALF;
     static constexpr int SC = MASK + 128;
-    static constexpr int OUTIDS = SC + NS * 128;
-    static constexpr int BUF = OUTIDS + (IDSOUT ? 128 : 0);
+    static constexpr int BUF = SC + (SCALAR ? 128 : 0);
     static constexpr int IDS = S * BUF;
     static constexpr int TAIL = IDS + 128;
     static constexpr int WARP_SMEM = (TAIL + TAIL_ + 127) / 128 * 128;
@@ -50,13 +48,13 @@ struct GStreamCfg {
 struct GStreamArgs {
     const int32_t *rowptr, *col, *win;
     const uint32_t *mask;
-    const int32_t *run_begin;  // [n_runs + 1] part ranges, or null: a run per part
-    const int32_t *run_slot;   // [n_runs] or null
+    const int32_t *run_begin;  // [n_runs + 1] part ranges
+    const int32_t *run_slot;   // [n_runs]
     int64_t n_runs, H, n_nodes, F;
     int wide;
-    const void *X[2];          // gathered tiles: row id of head h at X + id * ld + h * F
+    const void *X;             // gathered rows: id's of head h at X + id * ld + h * F
     int64_t ld;
-    const float *sc[4];        // per-column scalars [H][n_nodes]
+    const float *sc;           // per-column scalars [H][n_nodes] (SCALAR)
     int32_t *err;
 };
 
@@ -124,14 +122,9 @@ struct GatStream {
         r_slot = -1;
         if (item < n_items) {
             const int run = H == 1 ? item : item / H;
-            if (A.run_begin) {
-                r_p0 = __ldg(A.run_begin + run);
-                r_p1 = __ldg(A.run_begin + run + 1);
-                r_slot = __ldg(A.run_slot + run);
-            } else {
-                r_p0 = run;
-                r_p1 = run + 1;
-            }
+            r_p0 = __ldg(A.run_begin + run);
+            r_p1 = __ldg(A.run_begin + run + 1);
+            r_slot = __ldg(A.run_slot + run);
         }
     }
     struct Part {
@@ -247,9 +240,7 @@ struct GatStream {
             for (int k = 0; k < (C::RPL < 4 ? C::RPL : 4); ++k) {
                 const bool ok = WHOLE || id[k] >= 0;
                 const IT o = ok ? base + (IT)id[k] * ld : (IT)0;
-#pragma unroll
-                for (int t = 0; t < C::TILES; ++t)
-                    cp_async16(at(k0 + k) + t * C::TILE, (const T *)A.X[t] + o, ok ? 16 : 0);
+                cp_async16(at(k0 + k), (const T *)A.X + o, ok ? 16 : 0);
             }
         }
     }
@@ -272,16 +263,12 @@ struct GatStream {
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sbase + C::MASK + wbuf + 4 * lane),
                              "l"(ok ? m : reinterpret_cast<const char *>(A.mask)), "r"(ok ? 4 : 0));
             }
-            if constexpr (C::NS > 0) {
+            if constexpr (C::SCALAR) {
                 const bool ok = pid >= 0;
                 const IT o = (IT)p.h * (IT)A.n_nodes + (ok ? pid : 0);
-#pragma unroll
-                for (int k = 0; k < C::NS; ++k)
-                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sbase + C::SC + wbuf + k * 128 + 4 * lane),
-                                 "l"(A.sc[k] + o), "r"(ok ? 4 : 0));
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(sbase + C::SC + wbuf + 4 * lane),
+                             "l"(A.sc + o), "r"(ok ? 4 : 0));
             }
-            if constexpr (C::IDSOUT)
-                asm volatile("st.shared.b32 [%0], %1;\n" ::"r"(sbase + C::OUTIDS + wbuf + 4 * lane), "r"(pid) : "memory");
         }
         cp_async_commit();
     }
