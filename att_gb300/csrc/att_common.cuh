@@ -146,10 +146,9 @@ __device__ __forceinline__ void mma_1688_tf32(float (&d)[4], uint32_t a0, uint32
 // with truncation: hi keeps the sign, exponent and top 10 mantissa bits of x,
 // lo is the remainder x - hi (exact in fp32) truncated the same way, so
 // |x - hi - lo| < 2^-20 |x|.  The tensor core itself reads a .tf32 operand
-// without its low 13 bits (4 M products of random operands, denormals,
-// infinities and NaNs among them, came out bit-identical with and without them
-// masked off), so the operands are x and x - hi as they are: one logic
-// operation and one subtraction instead of two and one.
+// without its low 13 bits (a test holds it to that bit for bit, over random
+// bit patterns of every exponent), so the operands are x and x - hi as they are:
+// one logic operation and one subtraction instead of two and one.
 __device__ __forceinline__ void split_tf32x3(float x, uint32_t &hi, uint32_t &lo) {
     hi = __float_as_uint(x);
     lo = __float_as_uint(x - __uint_as_float(hi & 0xffffe000u));

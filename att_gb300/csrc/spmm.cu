@@ -594,8 +594,8 @@ __global__ void __launch_bounds__(kThreads) k_spmm16_tma(
 // each brings four features of one row, the m = gid and gid + 8 elements of
 // two feature tiles, so a tile's rows are features 4 gid + 2 v (+ 1) and a lane
 // ends up with four adjacent features of its window rows: one float4 store.
-// 169,343 nodes, mean degree 14, F = 100: 178 us, 9.4 TB/s into the SMs; with
-// one 4-byte load per fragment element in a per-step ring it took 369 us.
+// 169,343 nodes, mean degree 14, F = 100: 184 us a call, 9.4 TB/s into the SMs;
+// with one 4-byte load per fragment element in a per-step ring it took 388.
 template <int W, int FC, int WIDE, int S>
 struct CfgTF32 : StreamCfg<FC * 4, 4, W, WIDE, S, (W == 16 ? 12 : 20)> {
     static constexpr int MT = FC / 16;
@@ -1805,8 +1805,8 @@ constexpr int kTmaStages = 5;
 //    two; 4: three) and features per work item for F > 64 (a thread's 64 or 128 and
 //    a process-wide 128 are taken as they are; the process-wide 64, the default,
 //    leaves the choice to wide_items).  Three buffers gain nothing: 2.45M
-//    nodes, F = 128, 64 features x 2 buffers 1,734 us, x 3 1,722; 128 x 2 1,549,
-//    x 3 1,613.
+//    nodes, F = 128, 64 features x 2 buffers 1,727 us, x 3 1,737; 128 x 2 1,555,
+//    x 3 1,667.
 //  * spmm_fp8: 1 = A fragments dequantized in registers (k_spmm_fp8r, 128
 //    features per item when F > 64), 0 = through an fp16 shared tile
 //    (k_spmm_fp8).
@@ -1959,8 +1959,8 @@ int dispatch_fc32(const int32_t *rowptr, const int32_t *col, const void *val, co
                                          Y, m_out, ldy, err, st)
     // shapes (features per item x chunk buffers): 0, 3 = 64 x 2, 1 = 32 x 2,
     // 2 = 32 x 3 (F <= 32 always takes 32-feature items).  169,343 nodes, mean
-    // degree 14, us for shapes 0, 1, 2: F 64 104, 115, 123; F 100 200, 211, 225;
-    // F 128 181, 201, 215
+    // degree 14, us for shapes 0, 1, 2: F 64 92, 103, 121; F 100 184, 195, 230;
+    // F 128 171, 191, 226 (rows of 400 bytes do not start on 128-byte lines)
     if (F <= 32 || opt(kOptTf32) == 1 || opt(kOptTf32) == 2) {
         if (opt(kOptTf32) == 2) ATT_LTF(32, 3);
         ATT_LTF(32, 2);
