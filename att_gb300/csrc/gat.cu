@@ -245,7 +245,8 @@ __global__ void k_slot_edges(SlotEdgeArgs A) {
 // of the window in every block -- no divisions, one accumulator per head, the
 // map read once for all heads (it is the largest input: 81 MB against 20 MB of
 // edge values at 169,343 nodes) and four blocks in flight.  That graph, 4 heads:
-// row sums 534 -> 99 us, slot scores 486 -> 158, dense values 205 -> 66
+// row sums 534 -> 108 us (split windows merged), slot scores 486 -> 158, dense
+// values 205 -> 66
 // against a warp (or thread) per part and head with runtime divisions.
 constexpr int kQuad = 4;
 constexpr int kQUnroll = 4;

@@ -1,5 +1,5 @@
 """Torch-level GAT operators over the C ABI (att_node_scores, att_slot_edges,
-att_sddmm, att_gather_slot_values, att_rowsum, att_spmm).
+att_sddmm, att_gather_slot_values, att_rowsum_ordered, att_spmm).
 
 They work on the GAT block format: the row-window structure of the
 conversion plus a slot -> CSR-edge map.  The map handed to these functions is
