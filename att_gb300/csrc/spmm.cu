@@ -1216,7 +1216,8 @@ struct BatchStream {
             job_begin = warp_uniform((int)jobs[job].item_begin);
             job_end = job + 1 < n_jobs ? warp_uniform((int)jobs[job + 1].item_begin) : n_items;
         }
-        const int nch = warp_uniform(((int)jobs[job].F + FC - 1) / FC);
+        // counted in 64 bits: a width that does not fit is skipped further on
+        const int nch = warp_uniform((int)((jobs[job].F + FC - 1) / FC));
         const int local = item - job_begin;
         r_job = job;
         r_g = nch == 1 ? local : local / nch;
