@@ -52,6 +52,10 @@ _SIGNATURES = {
     "att_spmm": (_c_int, [_c_vp, _c_vp, _c_vp, _c_int, _c_vp, _c_vp, _c_i64, _c_vp, _c_int,
                           _c_vp, _c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_i64, _c_int, _c_int,
                           _c_vp, _c_vp]),
+    "att_spmm_scratch_bytes": (_c_sz, [_c_i64, _c_int, _c_i64]),
+    "att_spmm_ordered": (_c_int, [_c_vp, _c_vp, _c_vp, _c_int, _c_vp, _c_vp, _c_i64, _c_vp, _c_int,
+                          _c_vp, _c_i64, _c_i64, _c_i64, _c_vp, _c_i64, _c_i64, _c_int, _c_int,
+                          _c_vp, _c_vp, _c_sz, _c_vp]),
     "att_node_scores_pair": (_c_int, [_c_vp, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64,
                                       _c_vp, _c_vp, _c_i64, _c_vp, _c_vp, _c_i64, _c_vp]),
     "att_node_scores": (_c_int, [_c_vp, _c_int, _c_i64, _c_i64, _c_i64, _c_i64, _c_i64, _c_vp,

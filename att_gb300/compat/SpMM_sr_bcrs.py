@@ -21,7 +21,7 @@ def _check(t, name):
 
 
 def _forward(row_offsets, col_indices, values, t_window_row, t_atomic, rhs_matrix, dimN, mOri,
-             x_dtype, wide, granule):
+             x_dtype, wide, granule, ordered=False):
     for t, n in ((row_offsets, "row_offsets"), (col_indices, "col_indices"), (values, "values"),
                  (t_window_row, "t_window_row"), (t_atomic, "t_atomic"),
                  (rhs_matrix, "rhs_matrix")):
@@ -36,7 +36,8 @@ def _forward(row_offsets, col_indices, values, t_window_row, t_atomic, rhs_matri
     if Fp != dimN:
         X = torch.nn.functional.pad(X, (0, Fp - dimN))
     Y = ops.spmm(row_offsets.contiguous(), col_indices.contiguous(), values.contiguous(),
-                 t_window_row.contiguous(), t_atomic.contiguous(), X, mOri, window=8, wide=wide)
+                 t_window_row.contiguous(), t_atomic.contiguous(), X, mOri, window=8, wide=wide,
+                 ordered=ordered)
     if Fp != dimN:
         Y = Y[:, :dimN].contiguous()
     return [Y]

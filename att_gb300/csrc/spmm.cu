@@ -129,7 +129,7 @@ __global__ void __launch_bounds__((Cfg16<W, FC, WIDE, S>::NW * 32), 1)
 #pragma unroll
         for (int t = 0; t < C::NT; ++t) acc[j][t][0] = acc[j][t][1] = acc[j][t][2] = acc[j][t][3] = 0.f;
 
-    Stream<C, 2, FC, IT, FULL> st(A, lane, warp, sbase, &queue);
+    Stream<C, 2, FC, IT, FULL, true> st(A, lane, warp, sbase, &queue);
     while (st.more()) {
         const Chunk c = st.next();
         if (c.left > 0) {
@@ -148,17 +148,17 @@ __global__ void __launch_bounds__((Cfg16<W, FC, WIDE, S>::NW * 32), 1)
         if (c.left > 32) continue;
         // ---- the part's last chunk: its W x FC tile ----
         const IT f0 = (IT)c.fc * FC + gid;
-        const bool add = c.win & 1;
-        if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
+        const Target to = target(c.win, W, Y, m_out, ldy, A.tiles, A.F);
+        if (to.add || A.wait) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
-                float *dst = Y + (r * ldy + f0);
-                if (r < m_out) {
+                const int64_t r = to.row0 + t * 8 + 2 * tig + h;
+                float *dst = to.base + (r * to.ld + f0);
+                if (r < to.limit) {
                     // Y is written once: a streaming store leaves L2 to the X rows
-                    if (add) {
+                    if (to.add) {
 #pragma unroll
                         for (int j = 0; j < 2 * C::MT; ++j)
                             if (FULL || f0 + 8 * j < st.F) red_add_f32(dst + 8 * j, acc[j / 2][t][h + 2 * (j & 1)]);
@@ -660,13 +660,13 @@ __global__ void __launch_bounds__((CfgTF32<W, FC, WIDE, S>::NW * 32), 1)
         st.release();
         if (c.left > 32) continue;
         const IT f0 = (IT)c.fc * FC + 4 * gid;
-        const bool add = c.win & 1;
+        const bool add = (c.win & 3) == kAdd;
         if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
+                const int64_t r = (int64_t)(c.win >> 2) * W + t * 8 + 2 * tig + h;
                 if (r >= m_out) continue;
                 float *dst = Y + (r * ldy + f0);
 #pragma unroll
@@ -1075,14 +1075,14 @@ __global__ void __launch_bounds__((CfgF8R<W, FC, WIDE>::NW * 32), 1)
         // epilogue: tile j, lane -> features f0 + 16 j + 2 gid (+1), window
         // rows t * 8 + 2 tig (+1); F is a multiple of 16, so both features of
         // a pair are inside F together
-        const bool add = c.win & 1;
+        const bool add = (c.win & 3) == kAdd;
         if (add || A.wait) griddep_wait();  // the window's rows are zeroed by then
         const IT f0 = (IT)c.fc * FC + 2 * gid;
 #pragma unroll
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t r = (int64_t)(c.win >> 1) * W + t * 8 + 2 * tig + h;
+                const int64_t r = (int64_t)(c.win >> 2) * W + t * 8 + 2 * tig + h;
                 if (r >= m_out) continue;
                 float *dst = Y + (r * ldy + f0);
 #pragma unroll
@@ -1642,6 +1642,113 @@ __global__ void k_zero_all(float *__restrict__ Y, int64_t m_out, int64_t F, int6
     else Y[r * ldy + f] = 0.f;
 }
 
+// Adds the tiles of split windows to Y (rows that the zero pass cleared): for each
+// run of three and more parts of one window, their tiles in part order with the
+// rounding errors kept beside the sum (Knuth's two-sum), as exactly as in fp64.  A
+// block looks at 256 parts and 64 float4s of their tiles.  Its four groups of 64
+// threads share the short runs that open there, a run each; a long one is cut into
+// four stretches (a hub has hundreds of parts, read eight at a time), whose sums
+// meet in order.
+// With red.add in the kernel itself the order in which parts end decides the last
+// bits of a split window's rows, and a layer that rounds them to 16 bits shows it
+// (its weight gradient varies by up to 6e-5 from run to run).  us a call without and with this: 169,343 nodes, F = 64 43,
+// 54; 472,772 nodes of degree 35, F = 128 323, 369; 2.45M nodes, F = 128 1,549, 1,714.
+// Bound by the latency of short chains: the tiles of the middle one are 122 MB, 46 us.
+struct TileSum {
+    float s[4] = {0.f, 0.f, 0.f, 0.f}, e[4] = {0.f, 0.f, 0.f, 0.f};
+    __device__ __forceinline__ void add(const float (&x)[4]) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float t = s[i] + x[i], b = t - s[i];
+            e[i] += (s[i] - (t - b)) + (x[i] - b);
+            s[i] = t;
+        }
+    }
+    // n tiles of `per` float4s, eight in flight
+    __device__ __forceinline__ void add(const float4 *src, int64_t n, int per) {
+        for (; n > 0; n -= 8, src += 8 * (int64_t)per) {
+            float4 v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u < n) v[u] = __ldcs(src + u * (int64_t)per);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (u < n) add({v[u].x, v[u].y, v[u].z, v[u].w});
+        }
+    }
+    // an infinite or NaN sum has no error term
+    __device__ __forceinline__ float get(int i) const { return isfinite(s[i]) ? s[i] + e[i] : s[i]; }
+};
+
+constexpr int kLongRun = 8;
+
+template <int W>
+__global__ void __launch_bounds__(256, 4) k_merge_tiles(const int32_t *__restrict__ win, const int32_t *__restrict__ atomic,
+                                                        int64_t n_parts, const float4 *__restrict__ tiles, int F,
+                                                        float *__restrict__ Y, int64_t m_out, int64_t ldy, int vec) {
+    __shared__ int s_win[256 + 32], s_short[256], s_long[256], s_n[2];
+    __shared__ TileSum part[3][64];
+    const int lane = threadIdx.x & 31, group = threadIdx.x >> 6, place = threadIdx.x & 63;
+    const int64_t p0 = (int64_t)blockIdx.x * 256, p = p0 + threadIdx.x;
+    const int w = p < n_parts ? __ldg(win + p) : -1;
+    const int before = p > 0 && p < n_parts ? __ldg(win + p - 1) : -1;
+    const bool split = p < n_parts && __ldg(atomic + p) != 0;
+    s_win[threadIdx.x] = w;
+    if (threadIdx.x < 32) s_win[256 + threadIdx.x] = p + 256 < n_parts ? __ldg(win + p + 256) : -1;
+    if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    if (split && w != before) {  // runs of one and two were added by the SpMM kernel
+        int n = 1;
+        while (n <= kLongRun && s_win[threadIdx.x + n] == w) ++n;
+        if (n > kLongRun) s_long[atomicAdd(&s_n[1], 1)] = threadIdx.x;
+        else if (n > 2) s_short[atomicAdd(&s_n[0], 1)] = threadIdx.x | n << 16;
+    }
+    __syncthreads();
+    griddep_wait();
+    const int per = W / 4 * F;  // float4s of a tile
+    const int o = blockIdx.y * 64 + place;
+    const bool live = o < per;
+    auto put = [&](const TileSum &t, int wq) {  // features 4 o .. 4 o + 3 of the tile
+        const int r = 4 * o / F;
+        const int64_t row = (int64_t)wq * W + r;
+        // added, not stored: parts of one window need not stand together in a small list
+        if (row >= 0 && row < m_out) put4(Y + row * ldy + (4 * o - r * F), true, vec, t.get(0), t.get(1), t.get(2), t.get(3));
+    };
+    for (int i = group; i < s_n[0]; i += 4) {
+        const int l = s_short[i] & 0xffff, n = s_short[i] >> 16;
+        if (!live) break;
+        TileSum t;
+        t.add(tiles + (p0 + l) * per + o, n, per);
+        put(t, s_win[l]);
+    }
+    for (int i = 0; i < s_n[1]; ++i) {
+        const int l = s_long[i], wq = s_win[l];
+        int64_t n = kLongRun + 1;
+        for (;;) {
+            const int64_t k = p0 + l + n + lane;
+            const unsigned other = ~__ballot_sync(0xffffffffu, k < n_parts && __ldg(win + k) == wq);
+            n += other ? __ffs(other) - 1 : 32;
+            if (other) break;
+        }
+        const int64_t k0 = n * group / 4, k1 = n * (group + 1) / 4;
+        TileSum t;
+        if (live) t.add(tiles + (p0 + l + k0) * per + o, k1 - k0, per);
+        if (group > 0) part[group - 1][place] = t;
+        __syncthreads();
+        if (group == 0 && live) {
+#pragma unroll
+            for (int g = 0; g < 3; ++g) {
+                const TileSum &u = part[g][place];
+                t.add(u.s);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) t.e[j] += u.e[j];
+            }
+            put(t, wq);
+        }
+        __syncthreads();
+    }
+}
+
 template <typename K>
 int occupancy_grid(K kernel, int smem, int64_t items) {
     int per_sm = 0;
@@ -1656,10 +1763,10 @@ int occupancy_grid(K kernel, int smem, int64_t items) {
 // that calls griddep_launch) still runs; it calls griddep_wait before it
 // touches what that one writes.
 template <typename... P, typename... Q>
-int launch_dependent(void (*kernel)(P...), int grid, int threads, int smem, cudaStream_t st, const char *what,
+int launch_dependent(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t st, const char *what,
                      const Q &...args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)threads);
     cfg.dynamicSmemBytes = (size_t)smem;
     cfg.stream = st;
@@ -1678,10 +1785,19 @@ struct KernelOf {
     static constexpr auto value = K;
 };
 
+template <int W>
+int merge_tiles(const int32_t *win, const int32_t *atomic, int64_t n_parts, const float *tiles, int64_t F, float *Y,
+                int64_t m_out, int64_t ldy, cudaStream_t st) {
+    const int vec = ldy % 4 == 0 && ((uintptr_t)Y & 15) == 0;
+    const dim3 grid((unsigned)((n_parts + 255) / 256), (unsigned)((W / 4 * F + 63) / 64));
+    return launch_dependent(k_merge_tiles<W>, grid, 256, 0, st, "k_merge_tiles", win, atomic, n_parts,
+                            reinterpret_cast<const float4 *>(tiles), (int)F, Y, m_out, ldy, vec);
+}
+
 template <typename T, int W, int FC, int WIDE, int S>
 int launch16(const int32_t *rowptr, const int32_t *col, const void *val, const int32_t *win,
              const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
-             int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, cudaStream_t st) {
+             int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, float *tiles, cudaStream_t st) {
     using C = Cfg16<W, FC, WIDE, S>;
     const int n_chunks = (int)((F + FC - 1) / FC);
     const int64_t items = n_parts * n_chunks;
@@ -1695,8 +1811,9 @@ int launch16(const int32_t *rowptr, const int32_t *col, const void *val, const i
         const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
-        return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm16", A, Y, m_out, ldy);
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), tiles, err};
+        const int s = launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm16", A, Y, m_out, ldy);
+        return s != ATT_OK || !tiles ? s : merge_tiles<W>(win, atomic, n_parts, tiles, F, Y, m_out, ldy, st);
     };
     if (small && F % FC == 0) return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int32_t, true>>{});
     if (small) return run(KernelOf<k_spmm16<T, W, FC, WIDE, S, int32_t, false>>{});
@@ -1743,7 +1860,7 @@ int launch_tf32(const int32_t *rowptr, const int32_t *col, const void *val, cons
         const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
+        const StreamArgs A{rowptr, col, win, atomic, val, X, nullptr, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), nullptr, err};
         return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_tf32", A, Y, m_out, ldy, vec_out);
     };
     if (small) return run(KernelOf<k_spmm_tf32<W, FC, WIDE, S, int32_t>>{});
@@ -1882,7 +1999,7 @@ int launch_fp8r(const int32_t *rowptr, const int32_t *col, const void *val, cons
         const int prep = dynamic_smem<kernel>(C::SMEM);
         if (prep != ATT_OK) return prep;
         const int grid = (int)(items < sm_count() ? items : sm_count());
-        const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), err};
+        const StreamArgs A{rowptr, col, win, atomic, val, X, xscale, n_parts, n_x, F, ldx, n_chunks, zero_all(m_out, ldy), nullptr, err};
         return launch_dependent(kernel, grid, C::NW * 32, C::SMEM, st, "k_spmm_fp8r", A, Y, m_out, ldy, vec_out);
     };
     if (small && F % FC == 0) return run(KernelOf<k_spmm_fp8r<W, FC, WIDE, int32_t, true>>{});
@@ -1918,7 +2035,7 @@ inline int item_features(int64_t F, int64_t n_parts) {
 template <typename T, int W, int WIDE>
 int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, const int32_t *win,
                   const int32_t *atomic, int64_t n_parts, const void *X, int64_t n_x, int64_t F,
-                  int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err,
+                  int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int32_t *err, float *tiles,
                   cudaStream_t st) {
     // TMA row gathers for F >= 64 (the tensor map's 64-feature box fits); the
     // cp.async kernel for narrower features or an X without rows
@@ -1932,7 +2049,7 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
     }
     if (F <= 32)
         return launch16<T, W, 32, WIDE, 2>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
-                                        m_out, ldy, err, st);
+                                        m_out, ldy, err, tiles, st);
     if constexpr (W == 8 && WIDE == 8) {
         if (opt(kOptGather) == 2 && (F <= 64 || opt(kOptFc) != 128))
             return launch16_bulk<T, 3>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, Y,
@@ -1940,7 +2057,7 @@ int dispatch_fc16(const int32_t *rowptr, const int32_t *col, const void *val, co
     }
 #define ATT_L16S(FCv, Sv)                                                                       \
     return launch16<T, W, FCv, WIDE, Sv>(rowptr, col, val, win, atomic, n_parts, X, n_x, F, ldx, \
-                                         Y, m_out, ldy, err, st)
+                                         Y, m_out, ldy, err, tiles, st)
     if (item_features(F, n_parts) == 64) {
         if (opt(kOptStages) == 4) ATT_L16S(64, 3);
         ATT_L16S(64, 2);
@@ -1975,12 +2092,14 @@ int dispatch_fc32(const int32_t *rowptr, const int32_t *col, const void *val, co
 
 using namespace att;
 
-extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype,
-                        const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
-                        const void *X, int x_dtype, const float *x_scale, int64_t n_x_rows,
-                        int64_t F, int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int window,
-                        int wide, int32_t *err_flag, void *stream) {
-    clear_error();
+namespace att {
+namespace {
+
+// tiles: null, or att_spmm_scratch_bytes of scratch for the parts of split windows
+int spmm(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype, const int32_t *window_of_part,
+         const int32_t *atomic, int64_t n_parts, const void *X, int x_dtype, const float *x_scale, int64_t n_x_rows,
+         int64_t F, int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int window, int wide, int32_t *err_flag,
+         float *tiles, cudaStream_t st) {
     ATT_CHECK(n_parts >= 0 && m_out >= 0 && F >= 0 && n_x_rows >= 0, ATT_ERR_INVALID,
               "negative size");
     ATT_CHECK(window == 8 || window == 16, ATT_ERR_UNSUPPORTED, "window must be 8 or 16, got %d",
@@ -1989,8 +2108,8 @@ extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *v
     ATT_CHECK(ldy >= F, ATT_ERR_INVALID, "ldy %lld < F %lld", (long long)ldy, (long long)F);
     ATT_CHECK(n_parts == 0 || (rowptr && col && val && window_of_part && atomic && X),
               ATT_ERR_INVALID, "null format or X pointer");
-    cudaStream_t st = (cudaStream_t)stream;
     if (m_out == 0 || F == 0) return ATT_OK;
+    if (F > (1 << 20)) tiles = nullptr;  // k_merge_tiles: the grid's y, and 32-bit places in a tile
     int s = ATT_OK;
     {
         const int64_t threads = (n_parts + 1) * 8;
@@ -2018,7 +2137,7 @@ extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *v
         ATT_CHECK(ldx >= F, ATT_ERR_INVALID, "ldx < F");
 #define ATT_SPMM16(T, Wv, WIDEv)                                                             \
     return dispatch_fc16<T, Wv, WIDEv>(rowptr, col, val, window_of_part, atomic, n_parts, X, \
-                                       n_x_rows, F, ldx, Y, m_out, ldy, err_flag, st)
+                                       n_x_rows, F, ldx, Y, m_out, ldy, err_flag, tiles, st)
         if (val_dtype == ATT_F16) {
             if (window == 8 && wide == 8) ATT_SPMM16(__half, 8, 8);
             if (window == 8 && wide == 16) ATT_SPMM16(__half, 8, 16);
@@ -2084,6 +2203,37 @@ extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *v
     }
     set_error("unsupported (val_dtype=%d, x_dtype=%d) combination", val_dtype, x_dtype);
     return ATT_ERR_UNSUPPORTED;
+}
+
+}  // namespace
+}  // namespace att
+
+extern "C" int att_spmm(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype,
+                        const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
+                        const void *X, int x_dtype, const float *x_scale, int64_t n_x_rows,
+                        int64_t F, int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int window,
+                        int wide, int32_t *err_flag, void *stream) {
+    clear_error();
+    return spmm(rowptr, col, val, val_dtype, window_of_part, atomic, n_parts, X, x_dtype, x_scale, n_x_rows, F, ldx, Y,
+                m_out, ldy, window, wide, err_flag, nullptr, (cudaStream_t)stream);
+}
+
+extern "C" size_t att_spmm_scratch_bytes(int64_t n_parts, int window, int64_t F) {
+    if (n_parts <= 0 || window <= 0 || F <= 0) return 0;
+    return (size_t)n_parts * (size_t)window * (size_t)F * sizeof(float);
+}
+
+extern "C" int att_spmm_ordered(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype,
+                                const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts, const void *X,
+                                int x_dtype, const float *x_scale, int64_t n_x_rows, int64_t F, int64_t ldx, float *Y,
+                                int64_t m_out, int64_t ldy, int window, int wide, int32_t *err_flag, void *scratch,
+                                size_t scratch_bytes, void *stream) {
+    clear_error();
+    const size_t need = att_spmm_scratch_bytes(n_parts, window, F);
+    ATT_CHECK(need == 0 || (scratch && ((uintptr_t)scratch & 15) == 0 && scratch_bytes >= need), ATT_ERR_WORKSPACE,
+              "scratch of %zu bytes, %zu needed (16-byte aligned)", scratch_bytes, need);
+    return spmm(rowptr, col, val, val_dtype, window_of_part, atomic, n_parts, X, x_dtype, x_scale, n_x_rows, F, ldx, Y,
+                m_out, ldy, window, wide, err_flag, need ? (float *)scratch : nullptr, (cudaStream_t)stream);
 }
 
 extern "C" int att_set_option(const char *key, int value) {

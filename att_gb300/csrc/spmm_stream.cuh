@@ -77,6 +77,22 @@ __device__ __forceinline__ void put2(float *dst, bool add, bool vec, float a, fl
     }
 }
 
+// What the last chunk of a part does with its tile: stores it in the rows of its
+// window, adds it to them (split windows), or stores it in the part's own rows of
+// the tiles, which are added in part order later.  A window of two parts needs no
+// tiles: 0 + a + b is the same in either order.
+enum : int { kStore = 0, kAdd = 1, kTile = 2 };
+struct Target {
+    float *base;
+    int64_t row0, limit, ld;
+    bool add;
+};
+__device__ __forceinline__ Target target(int win, int W, float *Y, int64_t m_out, int64_t ldy, float *tiles, int64_t F) {
+    const int64_t row0 = (int64_t)(win >> 2) * W;
+    if ((win & 3) == kTile) return {tiles, row0, INT64_MAX, F, false};
+    return {Y, row0, m_out, ldy, (win & 3) == kAdd};
+}
+
 // RPL column ids from shared memory
 template <int RPL>
 __device__ __forceinline__ void lds_ids(int (&id)[RPL], uint32_t p) {
@@ -120,7 +136,7 @@ struct StreamCfg {
 struct Chunk {
     int start, left;  // first condensed column, real columns left in the part (0: an empty part)
     int fc;           // feature chunk, -1: no more items
-    int win;          // window * 2 + (split window)
+    int win;          // window * 4 + kStore / kAdd, or part * 4 + kTile
 };
 
 struct StreamArgs {
@@ -129,14 +145,16 @@ struct StreamArgs {
     const float *xscale;  // EXTRA: per-row scales
     int64_t n_parts, n_x, F, ldx;
     int n_chunks;
-    int wait;  // every row was zeroed: no store before that is done
+    int wait;      // every row was zeroed: no store before that is done
+    float *tiles;  // null, or [n_parts][W][F]: where parts of split windows are stored
     int32_t *err;
 };
 
 // IT: type of items and of X's row pitch in bytes -- int32_t when they fit
 // (the common case), else int64_t.  ESZ: bytes per feature; FC: features per
-// item; FULL: F is a multiple of FC.
-template <typename C, int ESZ, int FC, typename IT, bool FULL>
+// item; FULL: F is a multiple of FC; TILES: parts of split windows may go to tiles
+// (only where the kernel asks for it: in the e4m3 kernel the choice cost 9 %).
+template <typename C, int ESZ, int FC, typename IT, bool FULL, bool TILES = false>
 struct Stream {
     static_assert(FC * ESZ == C::XROW, "rows");
     const StreamArgs &A;
@@ -154,6 +172,7 @@ struct Stream {
     Chunk f;
     int fid;                       // the fetched chunk's ids, in flight
     int n_rp[3], n_win, n_atomic;  // of the next item, in flight until it is entered
+    int n_near;                    // with tiles: lane k < 5 the window of part k - 2 of it
     // copy cursor
     Chunk p;
     int pid;                       // the lane's id of the chunk (EXTRA)
@@ -197,11 +216,16 @@ struct Stream {
     }
     __device__ __forceinline__ void load_item() {
         n_rp[0] = n_rp[1] = n_rp[2] = n_win = n_atomic = 0;
+        if constexpr (TILES) n_near = -1;
         if (i_part < n_parts) {
 #pragma unroll
             for (int k = 0; k < 3; ++k) n_rp[k] = __ldg(A.rowptr + 2 * (int64_t)i_part + k);
             n_win = __ldg(A.win + i_part);
             n_atomic = __ldg(A.atomic + i_part);
+            if constexpr (TILES) {
+                const int64_t near = (int64_t)i_part + lane - 2;
+                if (A.tiles && lane < 5 && near >= 0 && near < A.n_parts) n_near = __ldg(A.win + near);
+            }
         }
     }
     __device__ __forceinline__ void fetch_ids() { fid = lane < f.left ? __ldg(A.col + f.start + lane) : -1; }
@@ -210,7 +234,12 @@ struct Stream {
         const PartInfo pi = part_check<C::WIDE>(n_rp[0], n_rp[1], n_rp[2], A.err);
         f.start = warp_uniform(pi.start);
         f.left = warp_uniform(pi.nreal);
-        f.win = warp_uniform(2 * n_win + (n_atomic != 0));
+        f.win = 4 * n_win + (n_atomic != 0 ? kAdd : kStore);
+        if (TILES && A.tiles) {  // three parts of one window in a row, this one among them
+            const unsigned b = __ballot_sync(0xffffffffu, n_near == n_win);
+            if (n_atomic != 0 && ((b & b >> 1 & b >> 2) & 7) != 0) f.win = 4 * (int)i_part + kTile;
+        }
+        f.win = warp_uniform(f.win);
         f.fc = i_part < n_parts ? i_fc : -1;
         set_item(warp_uniform(i_after));
         draw();

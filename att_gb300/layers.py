@@ -94,11 +94,14 @@ class GATInput:
 # GCN / GraphSAGE (end2end_ori/gcn_final/mgat_csr/mgat_conv.py:27-108)
 # ---------------------------------------------------------------------------
 def _spmm(inputInfo, X):
-    fn = SpMM_sr_bcrs.forward_fp16_gnn if inputInfo.precision == "fp16" else \
-        SpMM_sr_bcrs.forward_tf32_gnn
-    return fn(inputInfo.row_pointers, inputInfo.column_index, inputInfo.degrees,
-              inputInfo.t_window_rowTensor, inputInfo.t_atomicTensor, X.contiguous(),
-              inputInfo.num_nodes, X.size(1), inputInfo.num_nodes_ori)[0]
+    """The SpMM drop-in of the layer's precision; fp16 with split windows in one
+    order, because the layer rounds the sums to 16 bits and multiplies by them:
+    their last bits, where they varied, moved its weight gradient."""
+    kind = (torch.float16, 8, 8) if inputInfo.precision == "fp16" else (torch.float32, 4, 4)
+    return SpMM_sr_bcrs._forward(inputInfo.row_pointers, inputInfo.column_index, inputInfo.degrees,
+                                 inputInfo.t_window_rowTensor, inputInfo.t_atomicTensor,
+                                 X.contiguous(), X.size(1), inputInfo.num_nodes_ori, *kind,
+                                 ordered=True)[0]
 
 
 class MGCNFunction(torch.autograd.Function):

@@ -252,15 +252,24 @@ def set_launch_shape(shape):
     _tls.shape = None if shape is None else tuple(shape)
 
 
+# Up to this much scratch an ordered product keeps the tiles of split windows
+# apart (472,772 nodes at F = 128: 381 MB, 323 -> 369 us); beyond it (2.45M nodes
+# at F = 128: 1.7 GB, 1,549 -> 1,714 us) their parts are added as they end.
+_ORDERED_SCRATCH = 1 << 30
+
+
 def spmm(rowptr, col, val, window_of_part, atomic, X, m_out, window=8, wide=8, out=None,
-         x_scale=None, err_flag=None, shape=None):
+         x_scale=None, err_flag=None, shape=None, ordered=False):
     """Y[m_out, F] (fp32) = A_blocks X on tensor cores.
 
     X: [n_x, F] fp16 / bf16 (with matching ``val``), fp32 (3xTF32), or
     float8_e4m3fn with ``x_scale`` fp32 [n_x] (values fp16).  F must be a
     multiple of 8 (16-bit) or 4 (fp32); callers pad otherwise.  ``shape``: a
     launch shape returned by ``autotune.tune_spmm`` (the process-wide
-    defaults when None).
+    defaults when None).  ``ordered`` (16-bit features): the parts of split
+    windows are added in part order, so the result is the same bits in every run
+    (with up to 1 GiB of scratch; otherwise they are added in the order in which
+    they end).
     """
     set_launch_shape(shape)
     require_cuda()
@@ -276,9 +285,14 @@ def spmm(rowptr, col, val, window_of_part, atomic, X, m_out, window=8, wide=8, o
         raise ValueError("out must be fp32 with unit feature stride")
     ldy = int(out.stride(0)) if m_out > 1 else F
     n_parts = int(window_of_part.shape[0])
-    _lib.call("att_spmm", _p(rowptr), _p(col), _p(val), _DT[val.dtype], _p(window_of_part),
-              _p(atomic), n_parts, _p(X), _DT[X.dtype], _p(x_scale), n_x, F, ldx, _p(out),
-              m_out, ldy, window, wide, _p(err_flag), _stream())
+    args = (_p(rowptr), _p(col), _p(val), _DT[val.dtype], _p(window_of_part), _p(atomic), n_parts,
+            _p(X), _DT[X.dtype], _p(x_scale), n_x, F, ldx, _p(out), m_out, ldy, window, wide,
+            _p(err_flag))
+    if ordered and X.element_size() == 2 and 0 < (need := 4 * n_parts * window * F) <= _ORDERED_SCRATCH:
+        tiles = torch.empty(need, dtype=torch.uint8, device=X.device)
+        _lib.call("att_spmm_ordered", *args, _p(tiles), need, _stream())
+    else:
+        _lib.call("att_spmm", *args, _stream())
     return out
 
 

@@ -228,6 +228,17 @@ ATT_API int att_spmm(const int32_t *rowptr, const int32_t *col, const void *val,
              int64_t F, int64_t ldx, float *Y, int64_t m_out, int64_t ldy,
              int window, int wide, int32_t *err_flag, void *stream);
 
+/* The same product; of 16-bit features (with spmm_gather 0) the parts of split
+ * windows are stored in scratch and added in part order, as exactly as in fp64
+ * (att_spmm adds them to Y in the order in which they end): the same bits from run
+ * to run.  scratch: att_spmm_scratch_bytes(...) bytes, 16-byte aligned. */
+ATT_API size_t att_spmm_scratch_bytes(int64_t n_parts, int window, int64_t F);
+ATT_API int att_spmm_ordered(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype,
+             const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
+             const void *X, int x_dtype, const float *x_scale, int64_t n_x_rows, int64_t F,
+             int64_t ldx, float *Y, int64_t m_out, int64_t ldy, int window, int wide,
+             int32_t *err_flag, void *scratch, size_t scratch_bytes, void *stream);
+
 /* ======================================================================
  * GAT operators on the block format with a slot -> edge map (the format
  * att_block_fill writes with `map` / `map_t`).  They replace the
