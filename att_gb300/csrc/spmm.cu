@@ -666,7 +666,7 @@ __global__ void __launch_bounds__((CfgTF32<W, FC, WIDE, S>::NW * 32), 1)
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t r = (int64_t)(c.win >> 2) * W + t * 8 + 2 * tig + h;
+                const int64_t r = window_of(c.win) * W + t * 8 + 2 * tig + h;
                 if (r >= m_out) continue;
                 float *dst = Y + (r * ldy + f0);
 #pragma unroll
@@ -1082,7 +1082,7 @@ __global__ void __launch_bounds__((CfgF8R<W, FC, WIDE>::NW * 32), 1)
         for (int t = 0; t < C::NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const int64_t r = (int64_t)(c.win >> 2) * W + t * 8 + 2 * tig + h;
+                const int64_t r = window_of(c.win) * W + t * 8 + 2 * tig + h;
                 if (r >= m_out) continue;
                 float *dst = Y + (r * ldy + f0);
 #pragma unroll

@@ -87,8 +87,11 @@ struct Target {
     int64_t row0, limit, ld;
     bool add;
 };
+// a Chunk's win holds its window (or part) as 30 unsigned bits: an id of 2^29 and
+// more lies past the output, not before it
+__device__ __forceinline__ int64_t window_of(int win) { return (uint32_t)win >> 2; }
 __device__ __forceinline__ Target target(int win, int W, float *Y, int64_t m_out, int64_t ldy, float *tiles, int64_t F) {
-    const int64_t row0 = (int64_t)(win >> 2) * W;
+    const int64_t row0 = window_of(win) * W;
     if ((win & 3) == kTile) return {tiles, row0, INT64_MAX, F, false};
     return {Y, row0, m_out, ldy, (win & 3) == kAdd};
 }
@@ -234,10 +237,10 @@ struct Stream {
         const PartInfo pi = part_check<C::WIDE>(n_rp[0], n_rp[1], n_rp[2], A.err);
         f.start = warp_uniform(pi.start);
         f.left = warp_uniform(pi.nreal);
-        f.win = 4 * n_win + (n_atomic != 0 ? kAdd : kStore);
+        f.win = (int)(4u * (uint32_t)n_win + (n_atomic != 0 ? kAdd : kStore));
         if (TILES && A.tiles) {  // three parts of one window in a row, this one among them
             const unsigned b = __ballot_sync(0xffffffffu, n_near == n_win);
-            if (n_atomic != 0 && ((b & b >> 1 & b >> 2) & 7) != 0) f.win = 4 * (int)i_part + kTile;
+            if (n_atomic != 0 && ((b & b >> 1 & b >> 2) & 7) != 0) f.win = (int)(4u * (uint32_t)i_part + kTile);
         }
         f.win = warp_uniform(f.win);
         f.fc = i_part < n_parts ? i_fc : -1;
