@@ -2109,7 +2109,8 @@ int spmm(const int32_t *rowptr, const int32_t *col, const void *val, int val_dty
     ATT_CHECK(n_parts == 0 || (rowptr && col && val && window_of_part && atomic && X),
               ATT_ERR_INVALID, "null format or X pointer");
     if (m_out == 0 || F == 0) return ATT_OK;
-    if (F > (1 << 20)) tiles = nullptr;  // k_merge_tiles: the grid's y, and 32-bit places in a tile
+    // the grid of k_merge_tiles: 64 float4s of a tile a block, at most 65,535 blocks in y
+    if (F > 65535 * 64 / (window / 4)) tiles = nullptr;
     int s = ATT_OK;
     {
         const int64_t threads = (n_parts + 1) * 8;
