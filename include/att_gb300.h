@@ -231,7 +231,8 @@ ATT_API int att_spmm(const int32_t *rowptr, const int32_t *col, const void *val,
 /* The same product; of 16-bit features (with spmm_gather 0) the parts of split
  * windows are stored in scratch and added in part order, as exactly as in fp64
  * (att_spmm adds them to Y in the order in which they end): the same bits from run
- * to run.  scratch: att_spmm_scratch_bytes(...) bytes, 16-byte aligned. */
+ * to run.  Above 4,194,240 / (window / 4) features they are added as by att_spmm.
+ * scratch: att_spmm_scratch_bytes(...) bytes, 16-byte aligned. */
 ATT_API size_t att_spmm_scratch_bytes(int64_t n_parts, int window, int64_t F);
 ATT_API int att_spmm_ordered(const int32_t *rowptr, const int32_t *col, const void *val, int val_dtype,
              const int32_t *window_of_part, const int32_t *atomic, int64_t n_parts,
